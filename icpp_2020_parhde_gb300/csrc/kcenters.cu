@@ -362,11 +362,19 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
 // Batched Kcenters with one CTA per graph (batches of small graphs).  A grid-wide level barrier costs
 // more than a small graph's whole level, and every grid-wide level waits for the deepest graph of the
 // batch; here each CTA takes whole graphs from a work list (largest first) and runs their 3k passes with
-// block barriers only.  Per pass: a level-synchronous top-down BFS from the pass's source over queues in
-// the graph's own slice of the union's queue arrays -- a thread per frontier vertex, its neighbours' loads
-// issued in batches of eight before the claims (atomicCAS on the distance entry; appends through a
-// shared-memory counter) --, then the Kcenters fold over the graph's vertices (min distance,
-// farthest vertex with the lowest index on ties -- the key (min_d << 32) | ~v --, exact sum of squares).
+// block barriers only.  Per pass: a level-synchronous top-down BFS from the pass's source, then the Kcenters
+// fold over the graph's vertices (min distance, farthest vertex with the lowest index on ties -- the key
+// (min_d << 32) | ~v --, exact sum of squares).
+// What bounds a level is its chain of dependent accesses (frontier entry -> offsets -> adjacency -> claim ->
+// append), so everything but the CSR stays on the SM: the visited set is a bitmap in shared memory (claims are
+// shared-memory ORs), the frontier lists are in shared memory up to qcap entries and spill to the graph's slice
+// of the union's queues, distances are written once and never read back inside a level.  2^k lanes share a
+// frontier vertex, as many as leave the whole frontier in one round of the CTA.
+// Measured, 512 geometric graphs of 1k-200k vertices, 30 passes: 150 -> 49 ms (claims by a global compare-and-swap
+// per edge and queues in global memory before); the largest graph alone is 44 ms of it, 2.7 us a level: a round of
+// claims and appends by 32 warps about 1000 clocks, two DRAM trips (152 graphs at once do not fit L2) as much again.
+// Tried: 32-byte row records of 16-bit index differences in place of offsets and adjacency, 2-10 % slower (the
+// extra slots cost more instructions than the saved access).
 // Same outputs as the batched variant of kcenters_bfs_kernel: D columns over the union, sources, keys and
 // sums indexed [p * B + b].
 struct KbArgs {
@@ -381,21 +389,156 @@ struct KbArgs {
   int64_t *sources;
   int32_t *min_d;
   ull *sumsq;
-  uint32_t *q0, *q1;     // [N] each: frontier vertices
+  uint32_t *q0, *q1;     // [N] each: frontier vertices beyond qcap
+  uint32_t *vis;         // visited bitmaps in global memory when the largest graph's does not fit on the SM:
+  int64_t vis_stride;    // vis_stride words per CTA
+  int vis_words;         // shared memory: visited words, then two lists of qcap entries
+  uint32_t qcap;
   ull *edges;
   int *err;
 };
 
 constexpr int KB_THREADS = 1024;
 
+constexpr uint32_t KB_ROUND = 16;  // neighbours of a row per round: one round covers most rows of a geometric graph
+constexpr uint32_t KB_ROW = 256;  // neighbours of a row taken by its lane group; the rest by the whole warp
+
+extern __shared__ uint32_t kb_smem[];  // [vis_words] visited, then the two frontier lists
+
+struct KbLevel {
+  const uint32_t *gq_in;  // frontier: entry i in kb_smem[s_in + i] below qcap, else in gq_in
+  uint32_t *gq_out;
+  uint32_t *vis;          // visited bitmap when it is in global memory
+  uint32_t s_in, s_out;
+  unsigned *c;  // entries appended
+  int32_t *Dp;  // the graph's rows of the pass's column
+  const int64_t *off;  // the graph's rows
+  const uint32_t *adj;
+  uint32_t vb, cnt, qcap, src;
+  int32_t d;
+};
+
+// Shared-memory OR unless `skip`: a predicated instruction, no branch, so that several are in flight at once.
+// Returns the word before (all ones where skipped).
+__device__ __forceinline__ uint32_t shared_or_unless(uint32_t addr, uint32_t bits, uint32_t skip) {
+  uint32_t old;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %3, 0;\n\tmov.u32 %0, 0xffffffff;\n\t"
+      "@p atom.shared.or.b32 %0, [%1], %2;\n\t}"
+      : "=&r"(old)
+      : "r"(addr), "r"(bits), "r"(skip)
+      : "memory");
+  return old;
+}
+
+// Claim the warp's neighbours v[t] (graph-local; a visited vertex where a lane has none) and append the new ones.
+template <bool SV, int NB>
+__device__ __forceinline__ void kb_claim(const KbLevel &l, const uint32_t (&v)[NB]) {
+  const uint32_t *vis = SV ? kb_smem : l.vis;
+  const uint32_t vis_s = (uint32_t)__cvta_generic_to_shared(kb_smem);
+  const int lane = threadIdx.x & 31;
+  uint32_t word[NB], seen = 1;
+#pragma unroll
+  for (int t = 0; t < NB; t++) word[t] = *(const volatile uint32_t *)(vis + (v[t] >> 5));
+#pragma unroll
+  for (int t = 0; t < NB; t++) {
+    word[t] = __funnelshift_r(word[t], 0u, v[t]);  // shifted to the vertex's bit, here and below
+    seen &= word[t];
+  }
+  if (__all_sync(PHDE_FULL_MASK, seen)) return;
+#pragma unroll
+  for (int t = 0; t < NB; t++) {  // every OR issued before any of their results is used
+    if (SV)
+      word[t] = shared_or_unless(vis_s + (v[t] >> 5) * 4u, 1u << (v[t] & 31), word[t] & 1u);
+    else
+      word[t] = word[t] & 1u ? 0xffffffffu : atomicOr(l.vis + (v[t] >> 5), 1u << (v[t] & 31));
+  }
+  unsigned bal[NB], total = 0;
+#pragma unroll
+  for (int t = 0; t < NB; t++) {
+    word[t] = __funnelshift_r(word[t], 0xffffffffu, v[t]);
+    bal[t] = __ballot_sync(PHDE_FULL_MASK, !(word[t] & 1u));
+    total += __popc(bal[t]);
+  }
+  if (!total) return;
+  unsigned base = 0;
+  if (lane == 0) base = atomicAdd(l.c, total);
+  base = __shfl_sync(PHDE_FULL_MASK, base, 0);
+  const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+  for (int t = 0; t < NB; t++) {
+    if (!(word[t] & 1u)) {
+      const unsigned slot = base + __popc(bal[t] & below);
+      if (slot < l.qcap)
+        kb_smem[l.s_out + slot] = v[t];
+      else
+        l.gq_out[slot] = v[t];
+      l.Dp[v[t]] = l.d;
+    }
+    base += __popc(bal[t]);
+  }
+}
+
+// One level with G lanes per frontier vertex: up to KB_ROW of its neighbours by the lane group, 16 per round, then
+// the rest of long rows one row at a time by the whole warp.
+template <bool SV, int G>
+__device__ __forceinline__ void kb_level(const KbLevel &l) {
+  constexpr int NB = KB_ROUND / G;
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+  const uint32_t step = blockDim.x / G;
+  for (uint32_t i0 = (threadIdx.x & ~31u) / G; i0 < l.cnt; i0 += step) {
+    const uint32_t i = i0 + lane / G;
+    uint32_t u = l.src, deg = 0;
+    int64_t e0 = 0;
+    if (i < l.cnt) {
+      u = i < l.qcap ? kb_smem[l.s_in + i] : l.gq_in[i];
+      const int64_t *o = l.off + u;
+      e0 = __ldg(o);
+      deg = (uint32_t)(__ldg(o + 1) - e0);
+    }
+    const uint32_t *row = l.adj + e0;
+    const uint32_t own = min(deg, KB_ROW);
+    const uint32_t most = __reduce_max_sync(PHDE_FULL_MASK, own);
+    for (uint32_t r = 0; r < most; r += KB_ROUND) {
+      uint32_t v[NB];
+#pragma unroll
+      for (int t = 0; t < NB; t++) {
+        const uint32_t e = r + t * G + gl;
+        v[t] = e < own ? __ldg(row + e) - l.vb : u;
+      }
+      kb_claim<SV, NB>(l, v);
+    }
+    for (unsigned big = __ballot_sync(PHDE_FULL_MASK, gl == 0 && deg > KB_ROW); big; big &= big - 1) {
+      const int from = __ffs(big) - 1;
+      const uint32_t *brow = l.adj + __shfl_sync(PHDE_FULL_MASK, e0, from);
+      const uint32_t bd = __shfl_sync(PHDE_FULL_MASK, deg, from);
+      for (uint32_t r = KB_ROW; r < bd; r += 128) {
+        uint32_t v[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+          const uint32_t e = r + t * 32 + lane;
+          v[t] = e < bd ? __ldg(brow + e) - l.vb : u;
+        }
+        kb_claim<SV, 4>(l, v);
+      }
+    }
+  }
+}
+
+template <bool SV>
 __global__ void __launch_bounds__(KB_THREADS) kcenters_block_kernel(KbArgs a) {
   __shared__ int s_graph;
   // level L appends through s_c[L % 3]; after the level every thread reads it, and
   // thread 0 clears s_c[(L + 2) % 3] -- last read before this level's final barrier, next used two levels on
-  __shared__ ull s_c[3];
+  __shared__ unsigned s_c[3];
   __shared__ ull red[32];
   __shared__ int64_t s_src;
   const int tid = threadIdx.x;
+  KbLevel l;
+  uint32_t *vis = SV ? kb_smem : a.vis + (int64_t)blockIdx.x * a.vis_stride;
+  l.vis = vis;
+  l.qcap = a.qcap;
+  l.adj = a.adj;
   ull edges_local = 0;
   for (;;) {
     if (tid == 0) s_graph = (int)atomicAdd(a.next, 1u);
@@ -405,84 +548,91 @@ __global__ void __launch_bounds__(KB_THREADS) kcenters_block_kernel(KbArgs a) {
     if (gi >= a.B) break;
     const int b = a.order[gi];
     const int64_t vb = a.vbase[b], nb = a.vbase[b + 1] - vb;
-    int64_t src = vb;  // Kcenters starts at the graph's vertex 0
+    const int words = (int)((nb + 31) >> 5);
+    l.vb = (uint32_t)vb;
+    l.off = a.off + vb;
+    uint32_t src = 0;  // Kcenters starts at the graph's vertex 0
     for (int p = 0; p < a.P; p++) {
-      int32_t *Dp = a.D + (int64_t)p * a.N;
-      if (tid == 0) {
-        Dp[src] = 0;
-        a.q0[vb] = (uint32_t)src;
-        s_c[0] = 0ull;
-        s_c[1] = 0ull;
-      }
-      uint32_t cnt = 1;
-      const uint32_t *qin = a.q0 + vb;
-      uint32_t *qout = a.q1 + vb;
-      int32_t L = 0;
+      for (int w = tid; w < words; w += blockDim.x) vis[w] = 0u;
       __syncthreads();
-      while (cnt > 0) {
-        unsigned *c = (unsigned *)(s_c + (L % 3));
-        // a thread per frontier vertex; its neighbours in batches of 8 with every load of a batch in flight
-        // before the claims (a level's critical path is its chain of memory round trips)
-        for (uint32_t i = tid; i < cnt; i += blockDim.x) {
-          const uint32_t u = qin[i];
-          const int64_t e1 = a.off[u + 1];
-          for (int64_t e0 = a.off[u]; e0 < e1; e0 += 8) {
-            uint32_t vv[8];
-#pragma unroll
-            for (int t = 0; t < 8; t++) vv[t] = e0 + t < e1 ? __ldg(a.adj + e0 + t) : 0xffffffffu;
-            int old[8];  // all eight claims issued before any result is used
-#pragma unroll
-            for (int t = 0; t < 8; t++) old[t] = vv[t] != 0xffffffffu ? atomicCAS(Dp + vv[t], -1, L + 1) : 0;
-#pragma unroll
-            for (int t = 0; t < 8; t++) {
-              if (vv[t] == 0xffffffffu) continue;
-              edges_local++;
-              if (old[t] == -1) qout[atomicAdd(c, 1u)] = vv[t];
-            }
-          }
-        }
+      l.Dp = a.D + (int64_t)p * a.N + vb;
+      l.s_in = (uint32_t)a.vis_words;
+      l.s_out = (uint32_t)a.vis_words + a.qcap;
+      l.gq_in = a.q0 + vb;
+      l.gq_out = a.q1 + vb;
+      l.cnt = 1;
+      l.d = 0;
+      l.src = src;
+      edges_local += a.off[vb + nb] - a.off[vb];  // a connected graph's pass reads every row once
+      if (tid == 0) {
+        vis[src >> 5] = 1u << (src & 31);
+        l.Dp[src] = 0;
+        kb_smem[a.vis_words] = src;
+        s_c[0] = 0u;
+        s_c[1] = 0u;
+      }
+      int64_t reached = 1;
+      int ring = 0;
+      __syncthreads();
+      while (l.cnt > 0) {
+        l.c = s_c + ring;
+        l.d++;
+        if (l.cnt * 8 <= blockDim.x)
+          kb_level<SV, 8>(l);
+        else if (l.cnt * 4 <= blockDim.x)
+          kb_level<SV, 4>(l);
+        else
+          kb_level<SV, 2>(l);
         __syncthreads();
-        cnt = *c;
-        if (tid == 0) s_c[(L + 2) % 3] = 0ull;
-        const uint32_t *tq = qin;
-        qin = qout;
-        qout = (uint32_t *)tq;
-        L++;
+        l.cnt = *(volatile unsigned *)l.c;
+        reached += l.cnt;
+        if (tid == 0) s_c[ring == 0 ? 2 : ring - 1] = 0u;
+        ring = ring == 2 ? 0 : ring + 1;
+        const uint32_t s = l.s_in;
+        l.s_in = l.s_out;
+        l.s_out = s;
+        uint32_t *g = (uint32_t *)l.gq_in;
+        l.gq_in = l.gq_out;
+        l.gq_out = g;
+      }
+      if (reached < nb) {
+        if (tid == 0) atomicCAS(a.err, 0, PHDE_ERR_DISCONNECTED);
+        break;
       }
       // fold: min distance, farthest vertex (lowest index on ties), exact sum of squares
       ull kbest = 0, ssq = 0;
-      int bad = 0;
-      for (int64_t v = vb + tid; v < vb + nb; v += blockDim.x) {
-        const int32_t d = __ldcg(Dp + v);
-        if (d < 0) {
-          bad = 1;
-          continue;
+      int32_t *mind = a.min_d + vb;
+      for (int64_t v0 = tid; v0 < nb; v0 += 8 * (int64_t)blockDim.x) {
+        int32_t d[8], m[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          const int64_t v = v0 + t * (int64_t)blockDim.x;
+          d[t] = v < nb ? __ldcg(l.Dp + v) : 0;
+          m[t] = v < nb ? __ldcg(mind + v) : -1;
         }
-        ssq += (ull)d * (ull)d;
-        int32_t m = a.min_d[v];
-        if (d < m) {
-          m = d;
-          a.min_d[v] = m;
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          const int64_t v = v0 + t * (int64_t)blockDim.x;
+          if (v >= nb) continue;
+          ssq += (ull)d[t] * (ull)d[t];
+          if (d[t] < m[t]) mind[v] = m[t] = d[t];
+          const ull key = ((ull)(uint32_t)m[t] << 32) | (ull)(0xffffffffu - (uint32_t)(vb + v));
+          kbest = key > kbest ? key : kbest;
         }
-        const ull key = ((ull)(uint32_t)m << 32) | (ull)(0xffffffffu - (uint32_t)v);
-        kbest = key > kbest ? key : kbest;
       }
-      bad = __syncthreads_or(bad);
       ssq = block_sum(ssq, red);
       kbest = block_max_u64(kbest, red);
       if (tid == 0) {
         a.sumsq[(int64_t)p * a.B + b] = ssq;
-        a.sources[(int64_t)p * a.B + b] = src;
-        if (bad) atomicCAS(a.err, 0, PHDE_ERR_DISCONNECTED);
-        s_src = (int64_t)(0xffffffffu - (uint32_t)(kbest & 0xffffffffull));
+        a.sources[(int64_t)p * a.B + b] = vb + src;
+        s_src = (int64_t)(0xffffffffu - (uint32_t)(kbest & 0xffffffffull)) - vb;
       }
       __syncthreads();
-      src = s_src;
-      if (bad) break;
+      src = (uint32_t)s_src;
     }
+    __syncthreads();
   }
-  const ull etot = block_sum(edges_local, red);
-  if (tid == 0 && a.edges) atomicAdd(a.edges, etot);
+  if (tid == 0 && a.edges) atomicAdd(a.edges, edges_local);
 }
 
 __global__ void fill_i32_kernel(int32_t *p, int64_t n, int32_t v) {
@@ -621,7 +771,6 @@ int phde_run_bfs_batched_blocks(phde_ctx *ctx, int P, const int32_t *d_order, in
   uint32_t *q1 = (uint32_t *)phde_buf(ctx, "q.v1", sizeof(uint32_t) * N);
   unsigned *next = (unsigned *)phde_buf(ctx, "kb.next", sizeof(unsigned));
   if (!min_d || !q0 || !q1 || !next) return PHDE_ERR_OOM;
-  PHDE_CK(ctx, cudaMemsetAsync(d_D, 0xff, sizeof(int32_t) * (size_t)N * (size_t)P, ctx->stream));
   PHDE_CK(ctx, cudaMemsetAsync(next, 0, sizeof(unsigned), ctx->stream));
   int rc = phde_fill_i32(ctx, min_d, N, 0x7fffffff);
   if (rc) return rc;
@@ -642,10 +791,31 @@ int phde_run_bfs_batched_blocks(phde_ctx *ctx, int P, const int32_t *d_order, in
   a.q1 = q1;
   a.edges = d_edges;
   a.err = ctx->d_err;
-  int per_sm = 0;
-  PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kcenters_block_kernel, KB_THREADS, 0));
-  const int grid = std::max(1, std::min(B, ctx->nsm * std::max(per_sm, 1)));
-  kcenters_block_kernel<<<grid, KB_THREADS, 0, ctx->stream>>>(a);
+  // shared memory: the visited bitmap of the largest graph and two frontier lists; a bitmap that leaves no room
+  // for the lists moves to global memory.  One CTA of 1024 threads per SM: the largest graph's passes are the
+  // critical path, and a second CTA on its SM slows them (512 RGGs, 1k-200k vertices: 83.6 ms a layout with one,
+  // 106.6 ms with two of 512 threads, 100.1 ms with one of 512).
+  int64_t nmax = 0;
+  for (int b = 0; b < B; b++) nmax = std::max(nmax, ctx->batch_vbase[b + 1] - ctx->batch_vbase[b]);
+  const int64_t words = (nmax + 31) / 32;
+  int64_t room = (int64_t)(227 * 1024) - 1024 - 4 * words;
+  a.vis = nullptr;
+  a.vis_words = (int)words;
+  if (room < 8 * 1024) {
+    room = 64 * 1024;
+    a.vis_words = 0;
+  }
+  const int grid = std::min(B, ctx->nsm);
+  if (a.vis_words == 0) {
+    a.vis = (uint32_t *)phde_buf(ctx, "kb.vis", sizeof(uint32_t) * (size_t)words * grid);
+    if (!a.vis) return PHDE_ERR_OOM;
+  }
+  a.vis_stride = words;
+  a.qcap = (uint32_t)std::min<int64_t>(room / 8, 4096);
+  const size_t smem = sizeof(uint32_t) * ((size_t)a.vis_words + 2 * (size_t)a.qcap);
+  const auto kernel = a.vis ? kcenters_block_kernel<false> : kcenters_block_kernel<true>;
+  PHDE_CK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<grid, KB_THREADS, smem, ctx->stream>>>(a);
   PHDE_LAUNCHED(ctx);
   return PHDE_OK;
 }

@@ -197,3 +197,33 @@ def test_batched_other_options_match_single_layouts(precision, eig, k, c):
     xf, _ = cb.layout_batched(10, 2)  # the union view is back: the fused pipeline on the same batch
     for g, x in zip(gs, xf):
         assert x.shape == (g.n, 2) and np.all(np.isfinite(x))
+
+
+def broom(leaves: int, tail: int):
+    """A hub with `leaves` leaves and a path of `tail` vertices: one long row and one wide level."""
+    hub = np.zeros(leaves + 1, dtype=np.int64)
+    lo = np.concatenate([hub, np.arange(leaves + 1, leaves + tail, dtype=np.int64)])
+    hi = np.concatenate([np.arange(1, leaves + 2, dtype=np.int64), np.arange(leaves + 2, leaves + tail + 1, dtype=np.int64)])
+    return graphs._csr_from_undirected(leaves + tail + 1, lo, hi)
+
+
+@pytest.mark.parametrize("leaves", [255, 300, 4096, 6000, 1_900_000])
+def test_block_kcenters_row_list_and_bitmap_edges(monkeypatch, leaves):
+    """One CTA per graph against the whole-grid search where its rows, lists and bitmap reach their limits: a hub
+    row at and past the lane groups' 256 neighbours, a level at and past the lists' 4096 shared-memory entries,
+    a visited bitmap too large for shared memory; beside an ordinary graph.  The same layouts bit for bit."""
+    gs = [broom(leaves, 40), graphs.rgg(3000, dim=2, avg_degree=8, seed=51)]
+    out = {"union": {}, "blocks": {}}
+    for mode in ("union", "blocks") * 4:  # layouts are compared at the same autotuned segment length (rounding)
+        monkeypatch.setenv("PHDE_BATCH_BFS", mode)
+        with Context(0) as cb:
+            cb.upload_batch(gs)
+            xs, st = cb.layout_batched(4, 2)
+            out[mode][st["batch_seg_rows"]] = [x.copy() for x in xs]
+        common = set(out["union"]) & set(out["blocks"])
+        if common:
+            break
+    assert common
+    for rows in common:
+        for a, b in zip(out["union"][rows], out["blocks"][rows]):
+            assert np.array_equal(a, b)
