@@ -69,6 +69,7 @@ struct KcArgs {
   const int64_t *vbase;
   const int32_t *gid;
   ull *qinit;       // [1] level-0 queue counter of the pass (count << 32 | edges)
+  const int64_t *resume;  // passes kcenters_cluster_kernel finished, source of the next one (null: none)
 };
 
 // Per-graph fold of a batched pass: the max of `key` and the sum of `ssq` over the lanes of one graph
@@ -101,8 +102,17 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
   int64_t src = a.variant == 1 ? a.fixed_src[0] : 0;
   uint32_t step = 0;
   ull edges_local = 0;
+  int p0 = 0;
+  if (a.resume) {  // go on where the cluster stopped: the same history, from the passes' keys or sources
+    p0 = (int)a.resume[0];
+    if (p0 >= a.P) return;
+    src = a.resume[1];
+    for (int i = tid; i < p0; i += blockDim.x)
+      s_hist[i] = a.variant == 2 ? (uint32_t)a.sources[i] : 0xffffffffu - (uint32_t)(a.keys[i] & 0xffffffffull);
+    __syncthreads();
+  }
 
-  for (int p = 0; p < a.P; p++) {
+  for (int p = p0; p < a.P; p++) {
     int32_t *Dp = a.D + (int64_t)p * n;
     int64_t s_off = 0;
     uint32_t sdeg = 0;
@@ -635,6 +645,346 @@ __global__ void __launch_bounds__(KB_THREADS) kcenters_block_kernel(KbArgs a) {
   if (tid == 0 && a.edges) atomicAdd(a.edges, edges_local);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Kcenters on one thread-block cluster, for graphs whose levels are narrow (meshes, geometric graphs: hundreds of
+// levels of a few hundred vertices).  There a level of kcenters_bfs_kernel is a chain of latencies -- the grid
+// barrier, the frontier queue, offsets, adjacency, claim and append, each through L2 -- of about 4-5 us whatever
+// it finds.  Here the search state lives in the shared memory of the cluster's CTAs: 32-vertex words are dealt to
+// the CTAs in turn, the owner of a word keeps its visited word, two next-frontier words (the levels alternate) and
+// its rows' starts; a level is
+//   expand   the CTA's frontier vertices (a list in shared memory) send one remote OR per neighbour to the owner's
+//            next-frontier word -- no value returned, so nothing waits for it --;
+//   barrier  of the cluster (hardware, ~0.25 us), which also orders the ORs;
+//   scan     the owner takes next & ~visited of its words: new vertices, their distances and its next list.
+// Only the adjacency is read from L2.  Every CTA posts its frontier's size to all others before the barrier, so all
+// see the same total: 0 ends the pass, more than `limit` (a wide level: the whole grid is faster) leaves the
+// kernel, and kcenters_bfs_kernel, launched after it, goes on from the pass that was not finished.
+// Sources, history and duplicate fix-up as in kcenters_bfs_kernel; distances are unique, so the results are equal.
+// Measured (16 CTAs of 512 threads): a level is 3100 clocks on the 125 x 125 mesh (expand 840, barrier with the
+// ORs in flight 1240, scan 990), 4000 on a 150k-vertex 2-D geometric graph; whole layouts 21.4 -> 6.7 ms and
+// 139 -> 43 ms.  8 CTAs: 7.7 and 54 ms; 256 threads: 7.2 and 50 ms.
+struct KlArgs {
+  const int64_t *off;
+  const uint32_t *adj;
+  int64_t n;
+  int32_t *D;
+  int P, variant, require_all;
+  const int64_t *fixed_src;
+  int64_t *sources;
+  int32_t *min_d;
+  ull *sumsq, *keys, *edges;
+  int *err;
+  int64_t *resume;   // [2]: passes finished, source of the next one
+  int words;         // words owned by a CTA
+  int rows;          // row starts in shared memory
+  uint32_t limit;
+};
+
+constexpr int KL_THREADS = 512;
+constexpr int KL_MAX_CLUSTER = 16;
+constexpr uint32_t KL_LIST = 4096;   // frontier entries of a CTA; the limit of a level's total as well
+constexpr uint32_t KL_ROW = 512;     // longer rows are taken by the whole CTA
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The shared-memory address of CTA `rank`'s copy of a local address.
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void remote_or(uint32_t addr, uint32_t v) {
+  asm volatile("red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void remote_st32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void remote_st64(uint32_t addr, ull v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+}
+
+struct KlLevel {
+  const int64_t *off;
+  const uint32_t *adj;
+  const uint32_t *rs;    // row starts, 33 per word (null: from off)
+  const uint2 *list;     // the CTA's frontier: row start and length
+  uint32_t next;         // shared address of the level's next-frontier words
+  uint32_t cnt, rank, cmask, clog;
+};
+
+__device__ __forceinline__ uint32_t kl_vertex(const KlLevel &l, uint32_t x) {
+  return (((x >> 5) << l.clog | l.rank) << 5) | (x & 31);
+}
+__device__ __forceinline__ void kl_send(const KlLevel &l, uint32_t v) {
+  const uint32_t w = v >> 5;
+  remote_or(map_rank(l.next + ((w >> l.clog) << 2), w & l.cmask), 1u << (v & 31));
+}
+__device__ __forceinline__ uint2 kl_row(const KlLevel &l, uint32_t x) {
+  if (l.rs) {
+    const uint32_t *r = l.rs + (x >> 5) * 33 + (x & 31);
+    return make_uint2(r[0], r[1] - r[0]);
+  }
+  const int64_t *o = l.off + kl_vertex(l, x);
+  const int64_t e0 = __ldg(o);
+  return make_uint2((uint32_t)e0, (uint32_t)(__ldg(o + 1) - e0));
+}
+
+// Rows of at most KL_ROW neighbours with G lanes per frontier vertex, 16 neighbours per group and round.
+template <int G>
+__device__ __forceinline__ void kl_expand(const KlLevel &l, uint32_t &edges) {
+  constexpr int NB = 16 / G;
+  const uint32_t gl = threadIdx.x & (G - 1);
+  for (uint32_t i = threadIdx.x / G; i < l.cnt; i += KL_THREADS / G) {
+    const uint2 x = l.list[i];
+    const uint32_t deg = x.y;
+    if (deg > KL_ROW) continue;
+    if (gl == 0) edges += deg;
+    const uint32_t *row = l.adj + x.x;
+    for (uint32_t r = gl; r < deg; r += 16) {
+      uint32_t v[NB];
+#pragma unroll
+      for (int t = 0; t < NB; t++) v[t] = r + t * G < deg ? __ldg(row + r + t * G) : 0xffffffffu;
+#pragma unroll
+      for (int t = 0; t < NB; t++)
+        if (v[t] != 0xffffffffu) kl_send(l, v[t]);
+    }
+  }
+}
+
+// The cluster's maximum of every CTA's `mine` (thread 0's value counts); `slots` is a shared array of ranks.
+__device__ __forceinline__ ull cluster_max(ull mine, ull *slots, uint32_t rank, uint32_t C) {
+  if (threadIdx.x < C)
+    remote_st64(map_rank((uint32_t)__cvta_generic_to_shared(slots + rank), threadIdx.x), mine);
+  cluster_barrier();
+  ull m = 0;
+  for (uint32_t r = 0; r < C; r++) m = slots[r] > m ? slots[r] : m;
+  return m;
+}
+
+__global__ void __launch_bounds__(KL_THREADS) kcenters_cluster_kernel(KlArgs a) {
+  extern __shared__ uint32_t kl_smem[];  // list, visited, next[2], (row starts), history
+  __shared__ uint32_t s_counts[2][KL_MAX_CLUSTER];
+  __shared__ ull s_keys[KL_MAX_CLUSTER], s_sums[KL_MAX_CLUSTER], s_fix[KL_MAX_CLUSTER];
+  // of the two levels in turn: vertices listed, and whether a listed row is longer than KL_ROW
+  __shared__ uint32_t s_cnt[2], s_long[2];
+  __shared__ ull red[32];
+  const uint32_t tid = threadIdx.x, rank = cluster_rank(), C = cluster_size();
+  const int words = a.words, warp = tid >> 5, lane = tid & 31;
+  const int chunk = min(32, (words + KL_THREADS / 32 - 1) / (KL_THREADS / 32));  // words of a warp in one step of a scan
+  uint32_t *vis = kl_smem + 2 * KL_LIST, *next = vis + words;
+  uint32_t *rs = vis + 3 * words;
+  uint2 *list = (uint2 *)kl_smem;
+  uint32_t *hist = rs + (a.rows ? 33 * words : 0);
+  KlLevel l;
+  l.off = a.off;
+  l.adj = a.adj;
+  l.rs = a.rows ? rs : nullptr;
+  l.list = list;
+  l.rank = rank;
+  l.cmask = C - 1;
+  l.clog = 31 - __clz((int)C);
+  if (a.rows)
+    for (int i = tid; i < 33 * words; i += KL_THREADS) {
+      const int64_t v = ((((int64_t)(i / 33) << l.clog) | rank) << 5) + i % 33;
+      rs[i] = (uint32_t)a.off[v < a.n ? v : a.n];
+    }
+  const uint32_t next_s = (uint32_t)__cvta_generic_to_shared(next);
+  uint32_t edges = 0;
+  ull edges_all = 0;
+  int64_t src = a.variant == 1 ? a.fixed_src[0] : 0;
+  for (int p = 0; p < a.P; p++) {
+    int32_t *Dp = a.D + (int64_t)p * a.n;
+    for (int w = tid; w < 3 * words; w += KL_THREADS) vis[w] = 0u;
+    const bool mine = (((uint32_t)(src >> 5)) & l.cmask) == rank;
+    const uint32_t sx = (uint32_t)(((src >> 5) >> l.clog) << 5 | (src & 31));
+    if (tid == 0) s_long[1] = mine;
+    __syncthreads();
+    if (tid == 0 && mine) {
+      vis[sx >> 5] = 1u << (sx & 31);
+      list[0] = kl_row(l, sx);
+      Dp[src] = 0;
+    }
+    if (tid == 0 && rank == 0) a.sources[p] = src;
+    cluster_barrier();  // every CTA's words are clear
+    l.cnt = mine ? 1u : 0u;
+    uint32_t L = 0;
+    bool wide = false;
+    for (;;) {
+      const uint32_t par = L & 1;
+      l.next = next_s + par * 4u * words;
+      // ---- expand ----
+      if (tid == 0) {  // for the scan after the barrier; what the last scan left is in the other place
+        s_cnt[par] = 0u;
+        s_long[par] = 0u;
+      }
+      if (tid >= KL_THREADS - 32) {  // the last warp posts the count: it has no rows to expand in a narrow level
+        const uint32_t r = tid - (KL_THREADS - 32);
+        if (r < C) remote_st32(map_rank((uint32_t)__cvta_generic_to_shared(&s_counts[par][rank]), r), l.cnt);
+      }
+      if (l.cnt <= KL_LIST) {
+        if (l.cnt * 16 <= KL_THREADS)
+          kl_expand<16>(l, edges);
+        else if (l.cnt * 8 <= KL_THREADS)
+          kl_expand<8>(l, edges);
+        else
+          kl_expand<4>(l, edges);
+        if (s_long[par ^ 1]) {  // rows above KL_ROW, one at a time (set by the scan that listed them, or for the source)
+          for (uint32_t i = 0; i < l.cnt; i++) {
+            const uint2 x = list[i];
+            if (x.y <= KL_ROW) continue;
+            if (tid == 0) edges += x.y;
+            for (uint32_t e = tid; e < x.y; e += KL_THREADS) kl_send(l, __ldg(a.adj + x.x + e));
+          }
+        }
+      }
+      cluster_barrier();
+      const uint32_t total = __reduce_add_sync(PHDE_FULL_MASK, lane < (int)C ? s_counts[par][lane] : 0u);
+      if (total == 0) break;
+      if (total > a.limit) {
+        wide = true;
+        break;
+      }
+      // ---- scan: level L + 1 ----
+      L++;
+      // the new vertices of each word are listed by a warp together (a lane per bit): a wave that runs along the
+      // numbering fills whole words, and one thread per word took 2000-2700 clocks a level
+      uint32_t *nx = next + par * words;
+      for (int w0 = warp * chunk; w0 < words; w0 += (KL_THREADS / 32) * chunk) {
+        const int w = w0 + lane;
+        uint32_t nw = 0, slot = 0;
+        if (lane < chunk && w < words) {
+          nw = nx[w];
+          if (nw) {
+            nx[w] = 0u;
+            const uint32_t seen = vis[w];
+            nw &= ~seen;
+            vis[w] = seen | nw;
+            if (nw) slot = atomicAdd(&s_cnt[par], (uint32_t)__popc(nw));
+          }
+        }
+        bool longrow = false;
+        for (unsigned some = __ballot_sync(PHDE_FULL_MASK, nw != 0u); some; some &= some - 1) {
+          const int j = __ffs(some) - 1;
+          const uint32_t bits = __shfl_sync(PHDE_FULL_MASK, nw, j);
+          const uint32_t at = __shfl_sync(PHDE_FULL_MASK, slot, j) + __popc(bits & ((1u << lane) - 1u));
+          if (!((bits >> lane) & 1u)) continue;
+          const uint32_t y = ((uint32_t)(w0 + j) << 5) | lane;
+          Dp[kl_vertex(l, y)] = (int32_t)L;
+          if (at >= KL_LIST) continue;
+          const uint2 row = kl_row(l, y);
+          list[at] = row;
+          longrow |= row.y > KL_ROW;
+        }
+        if (longrow) s_long[par] = 1u;
+      }
+      __syncthreads();
+      l.cnt = *(volatile uint32_t *)&s_cnt[par];
+    }
+    edges_all += edges;
+    edges = 0;
+    if (wide) {  // leave the pass to the whole grid: its column as it was, the source to start from
+      for (int i = tid; i < 32 * words; i += KL_THREADS) {
+        const int64_t v = ((((int64_t)(i >> 5) << l.clog) | rank) << 5) | (i & 31);
+        if (v < a.n) Dp[v] = -1;
+      }
+      if (tid == 0 && rank == 0) {
+        a.resume[0] = p;
+        a.resume[1] = src;
+      }
+      break;
+    }
+    // ---- fold the CTA's vertices: min distance, farthest vertex, sum of squares ----
+    ull kbest = 0, ssq = 0;
+    int bad = 0;
+    for (int i0 = tid; i0 < 32 * words; i0 += 4 * KL_THREADS) {
+      int32_t d[4], m[4];
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        const int i = i0 + t * KL_THREADS;
+        const int64_t v = ((((int64_t)(i >> 5) << l.clog) | rank) << 5) | (i & 31);
+        const bool ok = i < 32 * words && v < a.n;
+        const bool seen = ok && ((vis[i >> 5] >> (i & 31)) & 1u);
+        if (ok && !seen) {
+          bad = 1;
+          Dp[v] = -1;
+        }
+        d[t] = seen ? __ldcg(Dp + v) : -1;
+        m[t] = seen && a.variant != 1 ? __ldcg(a.min_d + v) : 0;
+      }
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        if (d[t] < 0) continue;
+        const int i = i0 + t * KL_THREADS;
+        const int64_t v = ((((int64_t)(i >> 5) << l.clog) | rank) << 5) | (i & 31);
+        ssq += (ull)d[t] * (ull)d[t];
+        if (a.variant == 1) continue;
+        if (d[t] < m[t]) a.min_d[v] = m[t] = d[t];
+        const ull key = ((ull)(uint32_t)m[t] << 32) | (ull)(0xffffffffu - (uint32_t)v);
+        kbest = key > kbest ? key : kbest;
+      }
+    }
+    bad = __syncthreads_or(bad);
+    ssq = block_sum(ssq, red);
+    kbest = block_max_u64(kbest, red);
+    if (bad && (a.variant != 1 || a.require_all)) kbest = ~0ull;  // no key has every bit set
+    if (tid < C) remote_st64(map_rank((uint32_t)__cvta_generic_to_shared(s_sums + rank), tid), ssq);
+    const ull key = cluster_max(kbest, s_keys, rank, C);
+    if (key == ~0ull) {
+      if (tid == 0) atomicCAS(a.err, 0, PHDE_ERR_DISCONNECTED);
+      if (tid == 0 && rank == 0) a.resume[0] = a.P;
+      break;
+    }
+    if (tid == 0 && rank == 0) {
+      ull s = 0;
+      for (uint32_t r = 0; r < C; r++) s += s_sums[r];
+      a.sumsq[p] = s;
+      a.keys[p] = key;
+      a.resume[0] = p + 1;
+    }
+    if (p + 1 == a.P) break;
+    if (a.variant == 1) {
+      src = a.fixed_src[p + 1];
+      continue;
+    }
+    const uint32_t raw = 0xffffffffu - (uint32_t)(key & 0xffffffffull);
+    const int32_t maxval = (int32_t)(key >> 32);
+    int hit = 0;
+    for (int i = tid; i < p; i += KL_THREADS) hit |= hist[i] == raw;
+    hit = __syncthreads_or(hit);
+    int64_t nsrc = raw;
+    if (hit) {  // the highest-index vertex with the same minimum distance that is not in the history
+      ull best = 0;
+      for (int i = tid; i < 32 * words; i += KL_THREADS) {
+        const int64_t v = ((((int64_t)(i >> 5) << l.clog) | rank) << 5) | (i & 31);
+        if (v >= a.n || a.min_d[v] != maxval) continue;
+        bool inh = false;
+        for (int q = 0; q < p && !inh; q++) inh = hist[q] == (uint32_t)v;
+        if (!inh) best = (ull)v + 1ull;
+      }
+      best = block_max_u64(best, red);
+      best = cluster_max(best, s_fix, rank, C);
+      if (best) nsrc = (int64_t)(best - 1ull);
+    }
+    __syncthreads();
+    if (tid == 0) hist[p] = a.variant == 2 ? (uint32_t)src : raw;
+    src = nsrc;
+  }
+  cluster_barrier();  // no CTA leaves while another may still write to its shared memory
+  edges_all = block_sum(edges_all, red);
+  if (tid == 0 && a.edges) atomicAdd(a.edges, edges_all);
+}
+
 __global__ void fill_i32_kernel(int32_t *p, int64_t n, int32_t v) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = v;
 }
@@ -646,6 +996,66 @@ int phde_fill_i32(phde_ctx *ctx, int32_t *p, int64_t n, int32_t v) {
   if (blocks < 1) blocks = 1;
   fill_i32_kernel<<<blocks, 256, 0, ctx->stream>>>(p, n, v);
   PHDE_LAUNCHED(ctx);
+  return PHDE_OK;
+}
+
+// The passes on one cluster first, where the graph may have narrow levels and its bitmaps fit the cluster's shared
+// memory; *resume tells the whole-grid kernel what is left.  Average degree above KL_DEGREE: scale-free graphs,
+// whose second or third level is most of the graph.
+constexpr int64_t KL_DEGREE = 24;
+
+static int run_cluster_passes(phde_ctx *ctx, const KcArgs &g, const int64_t **resume) {
+  if (g.nnz > KL_DEGREE * g.n) return PHDE_OK;
+  const auto kernel = kcenters_cluster_kernel;
+  int C = KL_MAX_CLUSTER;
+  KlArgs a;
+  size_t smem = 0;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  cfg.blockDim = dim3(KL_THREADS);
+  cfg.stream = ctx->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  PHDE_CK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  for (;; C /= 2) {  // 16 CTAs, or 8 where the device cannot place 16
+    if (C < 8) return PHDE_OK;
+    a.words = (int)((g.W + C - 1) / C);
+    const size_t fixed = sizeof(uint2) * KL_LIST + sizeof(uint32_t) * (size_t)((g.P + 3) & ~3);
+    const size_t room = 224 * 1024;
+    a.rows = fixed + sizeof(uint32_t) * 36 * (size_t)a.words <= room;
+    smem = fixed + sizeof(uint32_t) * (a.rows ? 36 : 3) * (size_t)a.words;
+    if (smem > room) return PHDE_OK;
+    PHDE_CK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(C);
+    cfg.dynamicSmemBytes = smem;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit >= 1) break;
+    cudaGetLastError();
+  }
+  int64_t *res = (int64_t *)phde_buf(ctx, "kl.resume", sizeof(int64_t) * 2);
+  if (!res) return PHDE_ERR_OOM;
+  a.off = g.off;
+  a.adj = g.adj;
+  a.n = g.n;
+  a.D = g.D;
+  a.P = g.P;
+  a.variant = g.variant;
+  a.require_all = g.require_all;
+  a.fixed_src = g.fixed_src;
+  a.sources = g.sources;
+  a.min_d = g.min_d;
+  a.sumsq = g.sumsq;
+  a.keys = g.keys;
+  a.edges = g.edges;
+  a.err = g.err;
+  a.resume = res;
+  a.limit = KL_LIST;
+  PHDE_CK(ctx, cudaLaunchKernelEx(&cfg, kernel, a));
+  PHDE_LAUNCHED(ctx);
+  *resume = res;
   return PHDE_OK;
 }
 
@@ -741,6 +1151,8 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   a.beta = 18;
   void *args[] = {&a};
   cudaEventRecord(ctx->kev[0], ctx->stream);
+  a.resume = nullptr;
+  if (B == 0 && (rc = run_cluster_passes(ctx, a, &a.resume))) return rc;
   PHDE_CK(ctx, cudaLaunchCooperativeKernel((const void *)kcenters_bfs_kernel, dim3(ctx->nsm * per_sm),
                                            dim3(KC_THREADS), args, smem, ctx->stream));
   PHDE_LAUNCHED(ctx);

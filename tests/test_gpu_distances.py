@@ -187,3 +187,55 @@ def test_multi_source_bfs_on_mesh_and_disconnected(gpu_ctx):
     gpu_ctx.upload(g2)
     d = gpu_ctx.distances([0, 1, 3, 5])
     assert list(d[:, 0]) == [0, 1, 1, -1, -1, -1] and list(d[:, 2]) == [-1, -1, -1, 0, 1, 1]
+
+
+def _tree_of_levels(edges, n):
+    e = np.asarray(edges, dtype=np.int64)
+    return graphs._csr_from_undirected(n, e.min(axis=1), e.max(axis=1))
+
+
+def _two_stars(leaves: int, tail: int):
+    """Stars around A = 0 and B = 1, both joined to m = 2, which carries a path of `tail` vertices.  From a leaf the
+    stars' leaves are two levels apart; from the path's end they are one level of 2 * leaves vertices."""
+    e = [(0, 2), (1, 2)]
+    e += [(2 if i == 0 else 2 + i, 3 + i) for i in range(tail)]
+    first = 3 + tail
+    e += [(0, first + i) for i in range(leaves)] + [(1, first + leaves + i) for i in range(leaves)]
+    return _tree_of_levels(e, first + 2 * leaves)
+
+
+@pytest.mark.parametrize("make", [
+    lambda: graphs.path_graph(33),
+    lambda: graphs.mesh(37, 15, seed=7),                        # 17 words: most CTAs of the cluster own one
+    lambda: graphs.mesh(512, 3, seed=8),
+    lambda: _two_stars(511, 20),                                # rows at the whole-CTA threshold and past it
+    lambda: _two_stars(700, 20),
+    lambda: _two_stars(2048, 20),                               # 4096 vertices in one level: the cluster's limit
+    lambda: _two_stars(3000, 20),                               # past it in the second pass: the grid goes on
+    lambda: graphs.mesh(1000, 900, seed=9),                     # row starts no longer in shared memory
+], ids=["path33", "mesh37x15", "mesh512x3", "stars511", "stars700", "stars2048", "stars3000", "mesh1000x900"])
+@pytest.mark.parametrize("variant", [0, 2])
+def test_cluster_kcenters_exact_vs_oracle(gpu_ctx, make, variant):
+    """The searches on one thread-block cluster, and their continuation by the whole grid after a wide level: the
+    oracle's pivots and distances."""
+    g = make()
+    gpu_ctx.upload(g)
+    passes = 12
+    D, s = gpu_ctx.kcenters(passes, variant)
+    Do, so = orc.kcenters(g, passes, variant, parallel=True)
+    assert np.array_equal(s, so) and np.array_equal(D, Do)
+
+
+def test_cluster_kcenters_duplicate_sources_and_fixed_sources(gpu_ctx):
+    """More passes than vertices (the duplicate fix-up) and fixed sources, a vertex out of reach among them."""
+    g = graphs.path_graph(9)
+    gpu_ctx.upload(g)
+    D, s = gpu_ctx.kcenters(12, 0)
+    Do, so = orc.kcenters(g, 12, 0)
+    assert np.array_equal(s, so) and np.array_equal(D, Do)
+    two = _tree_of_levels([(i, i + 1) for i in range(60)] + [(61 + i, 62 + i) for i in range(10)], 72)
+    gpu_ctx.upload(two)
+    d = gpu_ctx.distances([5, 65])
+    assert np.array_equal(d[:, 0], orc.bfs(two, 5)) and np.array_equal(d[:, 1], orc.bfs(two, 65))
+    with pytest.raises(ParHDEError):
+        gpu_ctx.kcenters(3, 0)
