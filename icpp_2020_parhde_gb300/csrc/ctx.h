@@ -46,6 +46,7 @@ struct phde_ctx {
   int64_t ws_epoch = 0;                            // bumped whenever a workspace buffer is (re)allocated
   // SSSP band width: the mean edge weight of the uploaded graph (sssp.cu)
   double w_mean = 1.0;
+  int64_t w_maxdeg = 0;  // and the largest degree, which picks the kernel
   long long w_mean_epoch = -1;
   // drawing (draw.cu): the entry-row array's graph, and the size of the last image drawn
   long long draw_rows_epoch = -1;
