@@ -7,7 +7,7 @@
 // next-level frontier word.  Two ways to pick the vertices of a level:
 //   dense  -- every vertex not yet finished, in 32-vertex tiles: a `done` bitmap (saturated, both frontier
 //             words zero) lets a warp skip 32 finished vertices with one load;
-//   sparse -- when the frontier's out-edges are few (below nnz / 16): only the frontier's neighbours can
+//   sparse -- when the frontier's out-edges are few (below nnz / 32): only the frontier's neighbours can
 //             gain bits, so they are claimed once (a per-vertex level stamp), listed, and pulled; the
 //             stale output words of two levels back are cleared from their list.  The frontier of a
 //             sparse level is a (vertex, edge prefix) list that the previous level built (or that is
@@ -86,9 +86,8 @@ struct MsArgs {
   ull *trace;                 // optional [2*trace_cap]: per level end time (ns) and vertices given new bits
   int trace_cap;
   uint32_t *done;             // [n/32] bitmap: saturated with both frontier words zero (or a hub row): skipped
-  // [3][n/32] frontier bitmaps: bit v of fbm[L % 3] <=> vertex v's frontier word of level L is nonzero.  A pull
-  // tests a neighbour's bit (one L1/L2-resident word) before gathering its 32-byte word, so levels with a
-  // small frontier skip most gathers.  Level L reads fbm[L % 3], sets fbm[(L+1) % 3] and clears fbm[(L+2) % 3]
+  // [3][n/32] frontier bitmaps: bit v of fbm[L % 3] <=> vertex v's frontier word of level L is nonzero.  A
+  // saturated vertex whose own bit is clear is finished.  Level L reads fbm[L % 3], sets fbm[(L+1) % 3] and clears fbm[(L+2) % 3]
   // (read during level L-1, written again during level L+1).
   uint32_t *fbm[3];
   int win;                    // dense levels stage frontier windows in shared memory (MS_WIN)
@@ -130,23 +129,60 @@ __device__ __forceinline__ void ld_words(const ull *p, ull (&x)[W]) {
   }
 }
 
-// A neighbour's frontier words: from the shared-memory window when u lies in it (WIN), else through L2 --
-// after the frontier-bitmap test when use_bm (the window holds zero words for vertices outside the frontier).
-// Returns false when the words are known to be zero (not read).
-template <int W, bool WIN>
-__device__ __forceinline__ bool gather_front(const ull *fcur, const ull *swin, int64_t wlo, const uint32_t *fbm_cur,
-                                             bool use_bm, uint32_t u, ull (&x)[W], uint64_t keep) {
-  if constexpr (WIN) {
-    const uint64_t d = (uint64_t)((int64_t)u - wlo);
-    if (d < (uint64_t)(3 * MS_WIN)) {
+// The same where `on`, else zero words: predicated instructions and no branch, so that a batch of gathers is in
+// flight at once (with the load and the OR that waits for it under one branch, every gather of a row waited for
+// the one before it: a 32-row tile of a 3-D geometric graph took 31k clocks, most of it 12-22 such trips).
+template <int W>
+__device__ __forceinline__ void ld_front_if(const ull *p, ull (&x)[W], uint64_t keep, bool on) {
+  if constexpr (W == 4) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %6, 0;\n\tmov.u64 %0, 0;\n\tmov.u64 %1, 0;\n\tmov.u64 %2, 0;\n\t"
+        "mov.u64 %3, 0;\n\t@p ld.global.cg.L2::cache_hint.v4.u64 {%0, %1, %2, %3}, [%4], %5;\n\t}"
+        : "=&l"(x[0]), "=&l"(x[1]), "=&l"(x[2]), "=&l"(x[3])
+        : "l"(p), "l"(keep), "r"((uint32_t)on));
+  } else {
 #pragma unroll
-      for (int w = 0; w < W; w++) x[w] = swin[d * W + w];
-      return true;
-    }
+    for (int w = 0; w < W; w++)
+      asm volatile(
+          "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.u64 %0, 0;\n\t"
+          "@p ld.global.cg.L2::cache_hint.u64 %0, [%1], %2;\n\t}"
+          : "=&l"(x[w])
+          : "l"(p + w), "l"(keep), "r"((uint32_t)on));
   }
-  if (use_bm && !((__ldcg(fbm_cur + (u >> 5)) >> (u & 31)) & 1u)) return false;
-  ld_front<W>(fcur + (int64_t)u * W, x, keep);
-  return true;
+}
+
+// acc |= the frontier words of the NB neighbours u[j] with on[j] (u[j] is a vertex whether on or not).  WIN: from the
+// shared-memory window where they lie in it, which nearly all do (so one at a time, the others under a branch);
+// else through L2, all NB gathers in flight together.  Testing the neighbour's bit of the frontier bitmap before its
+// gather costs as many L2 requests as it saves, and a trip: 3-D geometric graph, 8M vertices, levels with 5-24 % of
+// the vertices in the frontier 700-740 us with the test, 445-480 without.
+template <int W, bool WIN, int NB>
+__device__ __forceinline__ void gather_fronts(const ull *fcur, const ull *swin, int64_t wlo, const uint32_t (&u)[NB],
+                                              const bool (&on)[NB], ull (&acc)[W], uint64_t keep) {
+  if constexpr (WIN) {
+#pragma unroll
+    for (int j = 0; j < NB; j++) {
+      if (!on[j]) continue;
+      ull x[W];
+      const uint64_t d = (uint64_t)((int64_t)u[j] - wlo);
+      if (d < (uint64_t)(3 * MS_WIN)) {
+#pragma unroll
+        for (int w = 0; w < W; w++) x[w] = swin[d * W + w];
+      } else {
+        ld_front<W>(fcur + (int64_t)u[j] * W, x, keep);
+      }
+#pragma unroll
+      for (int w = 0; w < W; w++) acc[w] |= x[w];
+    }
+  } else {
+    ull x[NB][W];
+#pragma unroll
+    for (int j = 0; j < NB; j++) ld_front_if<W>(fcur + (int64_t)u[j] * W, x[j], keep, on[j]);
+#pragma unroll
+    for (int j = 0; j < NB; j++)
+#pragma unroll
+      for (int w = 0; w < W; w++) acc[w] |= x[j][w];
+  }
 }
 
 // Record word for 4 sources: the 4 bits of `nib` select which of the four 16-bit lanes get value `val`.
@@ -219,7 +255,7 @@ __device__ __forceinline__ bool fbit(const uint32_t *bm, uint32_t u) { return (_
 
 template <int W, bool WIN = false>
 __device__ __forceinline__ void ms_pull_vertex(const MsArgs &a, const ull (&full)[W], const ull *fcur, ull *fnext,
-                                               const uint32_t *fbm_cur, uint32_t *fbm_next, bool use_bm, int32_t L,
+                                               const uint32_t *fbm_cur, uint32_t *fbm_next, int32_t L,
                                                int64_t v, bool act, int gl, bool mark_done, bool &newbits,
                                                uint32_t &deg, const ull *swin = nullptr, int64_t wlo = 0) {
   newbits = false;
@@ -247,19 +283,11 @@ __device__ __forceinline__ void ms_pull_vertex(const MsArgs &a, const ull (&full
   if (act && !sat)
     for (int64_t e = e0 + gl; e < e1; e += 2 * MS_GROUP) {
       const int64_t e2 = e + MS_GROUP;
-      const uint32_t u0 = ld_nc_hint(a.adj + e, stream);
-      const uint32_t u1 = e2 < e1 ? ld_nc_hint(a.adj + e2, stream) : u0;
-      // gather only the neighbours in this level's frontier (their bitmap bit): an empty word adds nothing
-      ull x0[W];
-      if (gather_front<W, WIN>(fcur, swin, wlo, fbm_cur, use_bm, u0, x0, keep)) {
-#pragma unroll
-        for (int w = 0; w < W; w++) acc[w] |= x0[w];
-      }
-      ull x1[W];
-      if (e2 < e1 && gather_front<W, WIN>(fcur, swin, wlo, fbm_cur, use_bm, u1, x1, keep)) {
-#pragma unroll
-        for (int w = 0; w < W; w++) acc[w] |= x1[w];
-      }
+      uint32_t u[2];
+      const bool on[2] = {true, e2 < e1};
+      u[0] = ld_nc_hint(a.adj + e, stream);
+      u[1] = on[1] ? ld_nc_hint(a.adj + e2, stream) : u[0];
+      gather_fronts<W, WIN, 2>(fcur, swin, wlo, u, on, acc, keep);
     }
 #pragma unroll
   for (int w = 0; w < W; w++)
@@ -282,16 +310,20 @@ __device__ __forceinline__ void ms_pull_vertex(const MsArgs &a, const ull (&full
 }
 
 // One light row v (neighbours e0 .. e1, at most MS_SMALL) pulled by one lane: the gathers four at a time, then
-// the finalisation (record nibbles by L2 reductions).  newbits: v got new bits; finished: v is saturated and
-// not in this level's frontier (its `done` bit may be set).
+// the finalisation.  s: v's seen words, which the caller loaded beside the row's
+// offsets; the next four neighbours are read while the gathers of the last four are in flight -- a level's time is
+// its chain of memory trips (17 of 28 cycles per issue waiting on loads, every throughput near 30 %).  newbits: v
+// got new bits; finished: v is saturated and not in this level's frontier (its `done` bit may be set).
 template <int W, bool WIN>
-__device__ __forceinline__ void ms_pull_light(const MsArgs &a, const ull (&full)[W], const ull *fcur, ull *fnext,
-                                              const uint32_t *fbm_cur, bool use_bm, int32_t L, int64_t v, int64_t e0,
-                                              int64_t e1, bool &newbits, bool &finished, const ull *swin,
+__device__ __forceinline__ void ms_pull_light(const MsArgs &a, const ull (&full)[W], const ull (&s)[W], const ull *fcur,
+                                              ull *fnext, const uint32_t *fbm_cur, int32_t L, int64_t v,
+                                              int64_t e0, int64_t e1, bool &newbits, bool &finished, const ull *swin,
                                               int64_t wlo) {
   newbits = finished = false;
-  ull s[W];
-  ld_words<W>(a.seen + v * W, s);
+  const uint64_t stream = l2_policy_evict_first(), keep = l2_policy_evict_last();
+  uint32_t u[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) u[j] = e0 + j < e1 ? ld_nc_hint(a.adj + e0 + j, stream) : 0u;
   bool sat = true;
 #pragma unroll
   for (int w = 0; w < W; w++) sat &= (s[w] == full[w]);
@@ -301,26 +333,25 @@ __device__ __forceinline__ void ms_pull_light(const MsArgs &a, const ull (&full)
     finished = !fbit(fbm_cur, (uint32_t)v);
     return;
   }
-  const uint64_t stream = l2_policy_evict_first(), keep = l2_policy_evict_last();
   ull acc[W];
 #pragma unroll
   for (int w = 0; w < W; w++) acc[w] = 0ull;
   for (int64_t e = e0; e < e1; e += 4) {
-    uint32_t u[4];
+    uint32_t un[4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) u[j] = e + j < e1 ? ld_nc_hint(a.adj + e + j, stream) : 0u;
+    for (int j = 0; j < 4; j++) un[j] = e + 4 + j < e1 ? ld_nc_hint(a.adj + e + 4 + j, stream) : 0u;
+    bool on[4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      ull x[W];
-      if (e + j < e1 && gather_front<W, WIN>(fcur, swin, wlo, fbm_cur, use_bm, u[j], x, keep)) {
+    for (int j = 0; j < 4; j++) on[j] = e + j < e1;
+    gather_fronts<W, WIN, 4>(fcur, swin, wlo, u, on, acc, keep);
 #pragma unroll
-        for (int w = 0; w < W; w++) acc[w] |= x[w];
-      }
-    }
+    for (int j = 0; j < 4; j++) u[j] = un[j];
   }
-  const unsigned val = (unsigned)(L + 2);  // level L+1, stored +1
-  ull *row = a.R ? (ull *)(a.R + v * a.RW + a.col0) : nullptr;
-  const uint64_t rec = l2_policy_evict_first();
+  // the record's entries (level L+1, stored +1) are written once each and by this lane alone: plain 16-bit stores,
+  // where 64-bit reductions of four entries fetch the sector they add to (8M-vertex 3-D geometric graph: 177 -> 150 ms
+  // a sweep).  Index-local graphs keep the reductions: their vertices get several neighbouring sources in one level
+  // (96 2-D graphs, learned: 28.2 ms a layout against 29.0 with 16-bit stores).
+  uint16_t *row = a.R ? a.R + v * a.RW + a.col0 : nullptr;
 #pragma unroll
   for (int w = 0; w < W; w++) {
     const ull nw = acc[w] & ~s[w];
@@ -328,12 +359,18 @@ __device__ __forceinline__ void ms_pull_light(const MsArgs &a, const ull (&full)
     if (nw) {
       newbits = true;
       a.seen[v * W + w] = s[w] | nw;
-      if (row)
-        for (ull m = nw; m;) {
-          const int gi = (__ffsll((long long)m) - 1) >> 2;
-          red_or_hint(row + 16 * w + gi, nibble_lanes((unsigned)(nw >> (4 * gi)) & 15u, val), rec);
-          m &= ~(15ull << (4 * gi));
+      if (row) {
+        if constexpr (WIN) {
+          for (ull m = nw; m;) {
+            const int gi = (__ffsll((long long)m) - 1) >> 2;
+            red_or_hint((ull *)row + 16 * w + gi, nibble_lanes((unsigned)(nw >> (4 * gi)) & 15u, (unsigned)(L + 2)),
+                        l2_policy_evict_first());
+            m &= ~(15ull << (4 * gi));
+          }
+        } else {
+          for (ull m = nw; m; m &= m - 1) row[64 * w + __ffsll((long long)m) - 1] = (uint16_t)(L + 2);
         }
+      }
     }
   }
 }
@@ -344,7 +381,7 @@ __device__ __forceinline__ void ms_pull_light(const MsArgs &a, const ull (&full)
 // shared-memory window starting at vertex wlo where they lie in it.
 template <int W, bool WIN>
 __device__ __forceinline__ void ms_dense_tile(const MsArgs &a, const ull (&full)[W], const ull *fcur, ull *fnext,
-                                              const uint32_t *fbm_cur, uint32_t *fbm_next, bool use_bm, int32_t L,
+                                              const uint32_t *fbm_cur, uint32_t *fbm_next, int32_t L,
                                               int64_t t, const ull *swin, int64_t wlo, ull &my_stat) {
   const int64_t n = a.n;
   const int lane = threadIdx.x & 31, gl = lane & (MS_GROUP - 1), grp = lane / MS_GROUP;
@@ -357,7 +394,11 @@ __device__ __forceinline__ void ms_dense_tile(const MsArgs &a, const ull (&full)
     const int64_t v = v0 + lane;
     const bool mine = (todo >> lane) & 1u;
     int64_t e0 = 0, e1 = 0;
+    ull s[W];
+#pragma unroll
+    for (int w = 0; w < W; w++) s[w] = 0ull;
     if (mine) {
+      ld_words<W>(a.seen + v * W, s);
       e0 = a.off[v];
       e1 = a.off[v + 1];
     }
@@ -365,7 +406,7 @@ __device__ __forceinline__ void ms_dense_tile(const MsArgs &a, const ull (&full)
     const unsigned lmask = __ballot_sync(PHDE_FULL_MASK, light);
     todo &= ~lmask;
     bool nb = false, fin = false;
-    if (light) ms_pull_light<W, WIN>(a, full, fcur, fnext, fbm_cur, use_bm, L, v, e0, e1, nb, fin, swin, wlo);
+    if (light) ms_pull_light<W, WIN>(a, full, s, fcur, fnext, fbm_cur, L, v, e0, e1, nb, fin, swin, wlo);
     const unsigned nbm = __ballot_sync(PHDE_FULL_MASK, nb), finm = __ballot_sync(PHDE_FULL_MASK, fin);
     if (lane == 0 && nbm) atomicOr(fbm_next + t, nbm);
     if (lane == 0 && finm) atomicOr(a.done + t, finm);
@@ -379,7 +420,7 @@ __device__ __forceinline__ void ms_dense_tile(const MsArgs &a, const ull (&full)
     const int64_t v = v0 + (act ? __ffs(rest) - 1 : 0);
     bool nb;
     uint32_t dv;
-    ms_pull_vertex<W, WIN>(a, full, fcur, fnext, fbm_cur, fbm_next, use_bm, L, v, act, gl, true, nb, dv, swin, wlo);
+    ms_pull_vertex<W, WIN>(a, full, fcur, fnext, fbm_cur, fbm_next, L, v, act, gl, true, nb, dv, swin, wlo);
     if (nb) my_stat += (1ull << 32) | (ull)dv;
     for (int j = 0; j < 32 / MS_GROUP && todo; j++) todo &= todo - 1u;
   }
@@ -478,9 +519,6 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
     // the frontier's totals: its list counter if the previous level built one, else its count
     const ull fstat = built_f ? __ldcg(a.lctr + sf) : __ldcg(a.lstat + sf);
     const uint32_t fedges = (uint32_t)(fstat & 0xffffffffull);
-    // test the frontier bitmap before each gather while the frontier holds at most a quarter of the vertices
-    // (above that, most neighbours are in it and the test only lengthens the dependent chain)
-    const bool use_bm = (int64_t)(fstat >> 32) <= n / 4;
     const bool sparse = (int64_t)fedges < a.sparse_edges;
     bool push = false;  // a sparse level that pushes (set below, uniform)
     if (sparse) {
@@ -616,7 +654,7 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
           const int64_t v = act ? (int64_t)a.cand[i] : 0;
           bool nb;
           uint32_t dv;
-          ms_pull_vertex<W>(a, full, fcur, fnext, fbm_cur, fbm_next, use_bm, L, v, act, gl, true, nb, dv);
+          ms_pull_vertex<W>(a, full, fcur, fnext, fbm_cur, fbm_next, L, v, act, gl, true, nb, dv);
           block_push(nb, (uint32_t)v, dv, a.qv[so], a.qe[so], a.lctr + so, &psc);
         }
       }
@@ -655,7 +693,7 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
           }
           __syncthreads();
           for (int64_t tt = t0 + warp; tt < t1; tt += nwarps)
-            ms_dense_tile<W, true>(a, full, fcur, fnext, fbm_cur, fbm_next, use_bm, L, tt, ms_dyn, wlo, my_stat);
+            ms_dense_tile<W, true>(a, full, fcur, fnext, fbm_cur, fbm_next, L, tt, ms_dyn, wlo, my_stat);
         }
       } else {
         // warps take MS_TILE_CHUNK tiles at a time from a level counter, so warps that meet heavy
@@ -669,7 +707,7 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
             if (t >= ntiles) break;
             tend = min(t + MS_TILE_CHUNK, ntiles);
           }
-          ms_dense_tile<W, false>(a, full, fcur, fnext, fbm_cur, fbm_next, use_bm, L, t, nullptr, 0, my_stat);
+          ms_dense_tile<W, false>(a, full, fcur, fnext, fbm_cur, fbm_next, L, t, nullptr, 0, my_stat);
         }
       }
     }
@@ -688,13 +726,15 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
       }
       if (sat) continue;  // the row's finalisation writes zero new bits either way
       const uint64_t stream = l2_policy_evict_first(), keep = l2_policy_evict_last();
-      for (int64_t e = e0 + lane; e < e1; e += 32) {
-        const uint32_t u = ld_nc_hint(a.adj + e, stream);
-        if (use_bm && !fbit(fbm_cur, u)) continue;
-        ull x[W];
-        ld_front<W>(fcur + (int64_t)u * W, x, keep);
+      for (int64_t e = e0 + lane; e < e1; e += 64) {
+        uint32_t u[2];
+        bool on[2];
 #pragma unroll
-        for (int w = 0; w < W; w++) acc[w] |= x[w];
+        for (int j = 0; j < 2; j++) {
+          on[j] = e + 32 * j < e1;
+          u[j] = on[j] ? ld_nc_hint(a.adj + e + 32 * j, stream) : 0u;
+        }
+        gather_fronts<W, false, 2>(fcur, nullptr, 0, u, on, acc, keep);
       }
 #pragma unroll
       for (int w = 0; w < W; w++) {
@@ -1018,7 +1058,7 @@ static int msbfs_run(phde_ctx *ctx, const int64_t *d_src, int nsrc, int nlist, i
     a.tctr = a.ccount + 2;
     a.stamp = stamp;
     a.cand = cand;
-    a.sparse_edges = std::max<int64_t>(ctx->nnz / 16, 1);
+    a.sparse_edges = std::max<int64_t>(ctx->nnz / 32, 1);
     a.levels_out = levels;
     a.trace = trace;
     a.trace_cap = trace_cap;
