@@ -190,14 +190,15 @@ __device__ __forceinline__ ull block_max_u64(ull v, ull *scratch) {
 // dv.  One 64-bit atomic per block advances both the slot count (high 32 bits) and the running edge
 // total (low 32 bits), so the start-edge array qe[] is non-decreasing in slot order -- that is what
 // lets the next top-down step find the owner of an edge by binary search.  Edge totals stay below
-// 2^32 because nnz < 2^32 (uint32 adjacency).  Must be called by every thread of the block.
+// 2^32 because nnz < 2^32 (uint32 adjacency).  qo, when given, takes a third word per slot.  Must be called by
+// every thread of the block.
 struct PushScratch {
   ull warp_tot[32];
   ull base;
 };
 
 __device__ __forceinline__ void block_push(bool flag, uint32_t v, uint32_t dv, uint32_t *qv, uint32_t *qe, ull *ctr,
-                                           PushScratch *sc) {
+                                           PushScratch *sc, uint32_t *qo = nullptr, uint32_t o = 0) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   const ull mine = flag ? ((1ull << 32) | (ull)dv) : 0ull;
   ull x = mine;
@@ -226,6 +227,7 @@ __device__ __forceinline__ void block_push(bool flag, uint32_t v, uint32_t dv, u
     uint32_t slot = (uint32_t)(pos >> 32);
     qv[slot] = v;
     qe[slot] = (uint32_t)(pos & 0xffffffffull);
+    if (qo) qo[slot] = o;
   }
   __syncthreads();
 }
