@@ -48,6 +48,8 @@ struct phde_ctx {
   double w_mean = 1.0;
   int64_t w_maxdeg = 0;  // and the largest degree, which picks the kernel
   long long w_mean_epoch = -1;
+  int eig_start = 0;               // start-vector values of the power iteration held by eig_start_buf (eigen.cu)
+  const void *eig_start_buf = nullptr;
   // drawing (draw.cu): the entry-row array's graph, and the size of the last image drawn
   long long draw_rows_epoch = -1;
   void *draw_rows_buf = nullptr;
