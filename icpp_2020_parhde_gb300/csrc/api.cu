@@ -66,7 +66,7 @@ __global__ void validate_csr_kernel(const int64_t *off, const uint32_t *adj, int
 
 // A barrier that waits for one more block than is launched: the bounded wait must give up.
 __global__ void barrier_timeout_kernel(GridSync *gs, int *err, uint64_t timeout_ns) {
-  grid_barrier(gs, err, timeout_ns, gridDim.x + 1);
+  grid_barrier<unsigned>(gs, err, timeout_ns, gridDim.x + 1, nullptr, nullptr);
 }
 
 // Published glibc TYPE_3 rand() stream (see eigen.cu); the reference draws random pivots with rand() % n.

@@ -155,8 +155,8 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
           block_push(b < a.B, v, dv, q0v, q0e, a.qinit, &psc, q0o, ov);
         }
       }
-      if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-      const ull q = __ldcg(a.qinit);
+      ull q;
+      if (!grid_sync_read(a.gs, a.err, a.timeout_ns, a.qinit, &q)) return;
       f_cnt = (uint32_t)(q >> 32);
       f_edges = (uint32_t)(q & 0xffffffffull);
     }
@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
           block_push(found, (uint32_t)v, dv, qout_v, qout_e, octr, &psc, qout_o, ov);
         }
       }
-      if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-      const ull out = __ldcg(octr);
+      ull out;
+      if (!grid_sync_read(a.gs, a.err, a.timeout_ns, octr, &out)) return;
       f_cnt = (uint32_t)(out >> 32);
       f_edges = (uint32_t)(out & 0xffffffffull);
       if (a.trace && blockIdx.x == 0 && tid == 0 && step < (uint32_t)a.trace_cap) {
@@ -346,13 +346,13 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
       if (tid == 0) atomicMax(a.keys + p, kbest);
     }
     if (p + 1 == a.P) break;
-    if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
+    ull key;
+    if (!grid_sync_read(a.gs, a.err, a.timeout_ns, a.keys + p, &key)) return;
 
     if (a.variant == 1) {
       src = a.fixed_src[p + 1];
       continue;
     }
-    const ull key = __ldcg(a.keys + p);
     const uint32_t raw = 0xffffffffu - (uint32_t)(key & 0xffffffffull);
     const int32_t maxval = (int32_t)(key >> 32);
     int hit = 0;
@@ -368,8 +368,8 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
         for (int i = 0; i < p && !inh; i++) inh = (s_hist[i] == (uint32_t)v);
         if (!inh) atomicMax(a.fixkey + p, (ull)v + 1ull);
       }
-      if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-      const ull fk = __ldcg(a.fixkey + p);
+      ull fk;
+      if (!grid_sync_read(a.gs, a.err, a.timeout_ns, a.fixkey + p, &fk)) return;
       if (fk) next = (int64_t)(fk - 1ull);
     }
     __syncthreads();

@@ -481,7 +481,10 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
   __shared__ ull s_stat;
   __shared__ unsigned s_tile;
   bool built_f = a.period == 0, built_z = true;  // lists of levels L-1 and L-2 exist (sparse levels build them)
-  if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
+  // the totals of the frontier of level L and of the one before it (their list counters, or the counts of dense
+  // levels), as the barrier that ended their level read them
+  ull fstat, zstat = 0;
+  if (!grid_sync_read(a.gs, a.err, a.timeout_ns, built_f ? a.lctr + 3 : a.lstat + 3, &fstat)) return;
   int32_t L = 0;
   for (;; L++) {
     if (L > 65533) {  // the 16-bit record holds levels up to 65534; every block sees the same L
@@ -516,8 +519,6 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
     }
     if (threadIdx.x == 0) s_stat = 0ull;
     ull my_stat = 0;  // dense: this thread's (count << 32 | edges) of vertices given new bits
-    // the frontier's totals: its list counter if the previous level built one, else its count
-    const ull fstat = built_f ? __ldcg(a.lctr + sf) : __ldcg(a.lstat + sf);
     const uint32_t fedges = (uint32_t)(fstat & 0xffffffffull);
     const bool sparse = (int64_t)fedges < a.sparse_edges;
     bool push = false;  // a sparse level that pushes (set below, uniform)
@@ -542,7 +543,7 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
       // mode: the array is fresh)
       if (a.lvl) {
       } else if (built_z) {
-        const uint32_t zcnt = (uint32_t)(__ldcg(a.lctr + sz) >> 32);
+        const uint32_t zcnt = (uint32_t)(zstat >> 32);
         for (int64_t i = gt; i < zcnt; i += gts) {
           const int64_t v = a.qv[sz][i];
 #pragma unroll
@@ -551,14 +552,14 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
       } else {
         for (int64_t i = gt; i < n * W; i += gts) fnext[i] = 0ull;
       }
-      if (!built_f && !grid_sync(a.gs, a.err, a.timeout_ns)) return;
+      ull fctr = fstat;
+      if (!built_f && !grid_sync_read(a.gs, a.err, a.timeout_ns, a.lctr + sf, &fctr)) return;
       // new bits can only appear next to the frontier: claim those neighbours once (stamp L+1), edge-balanced
       // over the frontier's edges, skipping finished vertices, and add up the candidates' degrees.  Then either
       // pull every candidate's neighbours (work in proportion to the candidates' edges) or, when those are
       // more than twice the frontier's -- hubs next to a small frontier, as in R-MAT's first levels -- push:
       // every frontier edge (u, v) ORs u's frontier word into v's accumulator (hacc, zero outside a level),
       // work in proportion to the frontier's edges but an L2 reduction per word.
-      const ull fctr = __ldcg(a.lctr + sf);
       const uint32_t fcnt = (uint32_t)(fctr >> 32), fe = (uint32_t)(fctr & 0xffffffffull);
       const uint32_t *fqv = a.qv[sf], *fqe = a.qe[sf];
       unsigned *cc = a.ccount + (L & 1);
@@ -597,9 +598,9 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
         slot0 = __shfl_sync(PHDE_FULL_MASK, slot0, 0);
         if (mine) a.cand[slot0 + __popc(bal & ((1u << lane) - 1u))] = v;
       }
-      if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-      const unsigned nc = __ldcg(cc);
-      push = __ldcg(ce) > 2ull * fe;  // uniform
+      unsigned nc;
+      if (!grid_sync_read(a.gs, a.err, a.timeout_ns, cc, &nc)) return;
+      push = block_read(ce) > 2ull * fe;  // uniform
       if (push) {
         for (int64_t base = gw * 32; base < fe; base += gws * 32) {
           const int64_t e = base + lane;
@@ -772,10 +773,12 @@ __global__ void __launch_bounds__(MS_THREADS, 2) msbfs_kernel(MsArgs a) {
       __syncthreads();
       if (threadIdx.x == 0 && s_stat) atomicAdd(a.lstat + so, s_stat);
     }
-    if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
+    ull ostat;
+    if (!grid_sync_read(a.gs, a.err, a.timeout_ns, sparse ? a.lctr + so : a.lstat + so, &ostat)) return;
     built_z = built_f;
     built_f = sparse;
-    const ull ostat = sparse ? __ldcg(a.lctr + so) : __ldcg(a.lstat + so);
+    zstat = fstat;
+    fstat = ostat;
     const unsigned tot = (unsigned)(ostat >> 32);
     if (a.trace && gt == 0 && L < a.trace_cap) {
       a.trace[2 * L] = global_timer_ns();

@@ -116,8 +116,8 @@ __global__ void __launch_bounds__(NA_THREADS) bfs_noalloc_kernel(NaArgs a) {
         block_push(found, (uint32_t)v, dv, qout_v, qout_e, octr, &psc);
       }
     }
-    if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-    const ull out = __ldcg(octr);
+    ull out;
+    if (!grid_sync_read(a.gs, a.err, a.timeout_ns, octr, &out)) return;
     f_cnt = (uint32_t)(out >> 32);
     f_edges = (uint32_t)(out & 0xffffffffull);
     if (in_bu) {

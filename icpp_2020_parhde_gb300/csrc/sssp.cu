@@ -221,15 +221,15 @@ __global__ void __launch_bounds__(SS_THREADS, MINB) sssp_nearfar_kernel(SsArgs a
         }
         cur ^= 1;
       }
-      if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-      const ull out = __ldcg(octr);
+      ull out;
+      if (!grid_sync_read(a.gs, a.err, a.timeout_ns, octr, &out)) return;
       f_cnt = (uint32_t)(out >> 32);
       f_edges = (uint32_t)(out & 0xffffffffull);
       it++;
       step++;
     }
     // ---- near frontier empty: move to the band of the closest far vertex ----
-    far_cnt = __ldcg(a.farctr + (phase & 1));
+    far_cnt = block_read(a.farctr + (phase & 1));
     if (far_cnt == 0) break;
     const uint32_t *far_in = (phase & 1) ? a.far1 : a.far0;
     uint32_t *far_out = (phase & 1) ? a.far0 : a.far1;
@@ -246,8 +246,8 @@ __global__ void __launch_bounds__(SS_THREADS, MINB) sssp_nearfar_kernel(SsArgs a
       *fout_ctr = 0u;
       a.minfar[(phase + 1) & 1] = ~0ull;
     }
-    if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-    const ull mf = __ldcg(mslot);
+    ull mf;
+    if (!grid_sync_read(a.gs, a.err, a.timeout_ns, mslot, &mf)) return;
     const int64_t T_old = T;
     if (mf != ~0ull) T = ((int64_t)mf / a.delta + 1) * (int64_t)a.delta;
     // split the pile: this is a step of its own, writing the next round's input queue
@@ -275,8 +275,8 @@ __global__ void __launch_bounds__(SS_THREADS, MINB) sssp_nearfar_kernel(SsArgs a
       }
       block_push2(to_near, v, dv, qout_v, qout_e, octr, keep, far_out, fout_ctr, &psc, qout_o, ov);
     }
-    if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-    const ull out = __ldcg(octr);
+    ull out;
+    if (!grid_sync_read(a.gs, a.err, a.timeout_ns, octr, &out)) return;
     f_cnt = (uint32_t)(out >> 32);
     f_edges = (uint32_t)(out & 0xffffffffull);
     it++;
@@ -413,13 +413,12 @@ __global__ void __launch_bounds__(SS_THREADS, MINB) sssp_group_kernel(SsArgs a) 
         }
         if (__syncthreads_or(nearm | farm)) block_push_r<R>(nearm, farm, v, ov, dv, qout, octr, far_in, fctr, &psc);
       }
-      if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-      f_cnt = __ldcg(octr);
+      if (!grid_sync_read(a.gs, a.err, a.timeout_ns, octr, &f_cnt)) return;
       it++;
       step++;
     }
     // ---- near frontier empty: move to the band of the closest far vertex (as in sssp_nearfar_kernel) ----
-    const unsigned far_cnt = __ldcg(a.farctr + (phase & 1));
+    const unsigned far_cnt = block_read(a.farctr + (phase & 1));
     if (far_cnt == 0) break;
     const uint32_t *far_in = (phase & 1) ? a.far1 : a.far0;
     uint32_t *far_out = (phase & 1) ? a.far0 : a.far1;
@@ -436,8 +435,8 @@ __global__ void __launch_bounds__(SS_THREADS, MINB) sssp_group_kernel(SsArgs a) 
       *fout_ctr = 0u;
       a.minfar[(phase + 1) & 1] = ~0ull;
     }
-    if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-    const ull mf = __ldcg(mslot);
+    ull mf;
+    if (!grid_sync_read(a.gs, a.err, a.timeout_ns, mslot, &mf)) return;
     const int64_t T_old = T;
     if (mf != ~0ull) T = ((int64_t)mf / a.delta + 1) * (int64_t)a.delta;
     uint4 *qout = (step & 1) ? q0 : q1;
@@ -463,8 +462,7 @@ __global__ void __launch_bounds__(SS_THREADS, MINB) sssp_group_kernel(SsArgs a) 
       block_push_r<1>(nearm, keepm, v, ov, dv, qout, octr, far_out, fout_ctr, &psc);
       __syncthreads();
     }
-    if (!grid_sync(a.gs, a.err, a.timeout_ns)) return;
-    f_cnt = __ldcg(octr);
+    if (!grid_sync_read(a.gs, a.err, a.timeout_ns, octr, &f_cnt)) return;
     it++;
     step++;
     phase++;
