@@ -56,6 +56,7 @@ struct KcArgs {
   uint32_t *bm[3];  // frontier bitmaps, W words each, rotating with the global step (zero initially)
   int64_t W;        // words per bitmap
   int smem_bm;      // copy the frontier bitmap into shared memory for bottom-up levels
+  int cap;          // entries of the block's list of new vertices: a multiple of KC_THREADS, at least two of them
   ull *ctr;         // [4] ring of (count << 32 | edges)
   ull *edges;       // [1] adjacency entries read
   ull *trace;       // optional timeline: per level {globaltimer, pass<<40 | level<<32 | in_bu, frontier count, edges}
@@ -92,12 +93,54 @@ __device__ __forceinline__ void batch_fold(ull *keys, ull *sumsq, int g, ull key
   }
 }
 
+// The vertices a block finds in a level wait in a shared-memory list (warp-aggregated appends) and go to the grid's
+// queue a block-width at a time: a push is two block barriers and a round trip to the queue's counter, 2700-3200
+// clocks, and one per iteration also kept the iterations' memory trips from overlapping.
+struct KcList {
+  uint32_t *v;
+  unsigned *n;
+  __device__ __forceinline__ void add(bool flag, uint32_t x) const {
+    const unsigned bal = __ballot_sync(PHDE_FULL_MASK, flag);
+    if (!bal) return;
+    const int lane = threadIdx.x & 31;
+    unsigned at = 0;
+    if (lane == 0) at = atomicAdd(n, (unsigned)__popc(bal));
+    at = __shfl_sync(PHDE_FULL_MASK, at, 0) + __popc(bal & ((1u << lane) - 1u));
+    if (flag) v[at] = x;
+  }
+  // every thread of the block; the list is empty after it
+  __device__ __forceinline__ void flush(const int64_t *off, uint32_t *qv, uint32_t *qe, uint32_t *qo, ull *ctr,
+                                        PushScratch *sc) const {
+    __syncthreads();
+    const unsigned c = *(volatile unsigned *)n;
+    if (c == 0) return;
+    for (unsigned i0 = 0; i0 < c; i0 += blockDim.x) {
+      const bool has = i0 + threadIdx.x < c;
+      uint32_t x = 0, o = 0, d = 0;
+      if (has) {
+        x = v[i0 + threadIdx.x];
+        const int64_t o0 = __ldg(off + x);
+        o = (uint32_t)o0;
+        d = (uint32_t)(__ldg(off + x + 1) - o0);
+      }
+      block_push(has, x, d, qv, qe, ctr, sc, qo, o);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *n = 0u;
+    __syncthreads();
+  }
+};
+
 __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
   __shared__ PushScratch psc;
+  __shared__ unsigned s_listed;
   __shared__ uint32_t s_win[KC_THREADS / 32][32];
   __shared__ ull red[32];
-  extern __shared__ uint32_t s_hist[];  // [P]: every block keeps the same selection history, then the bitmap
-  uint32_t *s_bm = s_hist + ((a.P + 3) & ~3);
+  extern __shared__ uint32_t s_hist[];  // [P]: every block keeps the same selection history; the list, the bitmap
+  const KcList list{s_hist + ((a.P + 3) & ~3), &s_listed};
+  uint32_t *s_bm = list.v + a.cap;
+  const int full = a.cap / KC_THREADS - 1;  // iterations between looks at the list
+  if (threadIdx.x == 0) s_listed = 0u;  // barriers of the first pass's start come before its use
   const int64_t n = a.n;
   const int tid = threadIdx.x;
   const int64_t gstride = (int64_t)gridDim.x * blockDim.x;
@@ -192,10 +235,11 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
 
       if (!in_bu) {
         const int64_t E = f_edges;
+        int since = 0;
         for (int64_t base = gbase; base < E; base += gstride) {
           const int64_t e = base + tid, e0w = base + (tid & ~31);
           bool claimed = false;
-          uint32_t v = 0, dv = 0, ov = 0;
+          uint32_t v = 0;
           if (e0w < E) {  // warp-uniform
             int64_t j = s_off + e;
             if (L != 0 || a.B != 0) {
@@ -206,29 +250,33 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
             if (e < E) {
               v = __ldg(a.adj + j);
               edges_local++;
-              if (Dp[v] == -1) {
-                const int64_t o0 = __ldg(a.off + v), o1 = __ldg(a.off + v + 1);  // in flight with the claim
-                if (atomicCAS(Dp + v, -1, L + 1) == -1) {
-                  claimed = true;
-                  ov = (uint32_t)o0;
-                  dv = (uint32_t)(o1 - o0);
-                  atomicOr(bm_next + (v >> 5), 1u << (v & 31));
-                }
+              if (Dp[v] == -1 && atomicCAS(Dp + v, -1, L + 1) == -1) {
+                claimed = true;
+                atomicOr(bm_next + (v >> 5), 1u << (v & 31));
               }
             }
+            list.add(claimed, v);
           }
-          block_push(claimed, v, dv, qout_v, qout_e, octr, &psc, qout_o, ov);
+          if (++since == full) {  // as many more as the list holds for sure
+            since = 0;
+            __syncthreads();
+            if (__syncthreads_or(s_listed > KC_THREADS)) list.flush(a.off, qout_v, qout_e, qout_o, octr, &psc);
+          }
         }
+        list.flush(a.off, qout_v, qout_e, qout_o, octr, &psc);
       } else {
         if (a.smem_bm) {
-          for (int64_t w = tid; w < a.W; w += blockDim.x) s_bm[w] = __ldcg(bm_cur + w);
+          // 16 bytes per copy, all of a thread's in flight (word by word: 11k clocks for R-MAT 20's 80 KB)
+          for (int64_t w = 4 * (int64_t)tid; w < a.W; w += 4 * (int64_t)blockDim.x) cp_async16(s_bm + w, bm_cur + w);
+          cp_async_commit();
+          cp_async_wait<0>();
           __syncthreads();
         }
         const uint32_t *front = a.smem_bm ? s_bm : bm_cur;
+        int since = 0;
         for (int64_t base = gbase; base < n; base += gstride) {
           const int64_t v = base + tid;
           bool found = false;
-          uint32_t dv = 0, ov = 0;
           if (v < n && Dp[v] == -1) {
             const int64_t j0 = a.off[v], j1 = a.off[v + 1];
             // four neighbours per round (their adjacency entries, then their bitmap words, all in flight): a
@@ -249,16 +297,20 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
             }
             if (found) {
               Dp[v] = L + 1;
-              ov = (uint32_t)j0;
-              dv = (uint32_t)(j1 - j0);
             }
           }
           // one bitmap word per warp: the warp covers 32 consecutive, 32-aligned vertices
           const uint32_t bal = __ballot_sync(PHDE_FULL_MASK, found);
           const int64_t v0 = v - (tid & 31);
           if ((tid & 31) == 0 && v0 < n) bm_next[v0 >> 5] = bal;
-          block_push(found, (uint32_t)v, dv, qout_v, qout_e, octr, &psc, qout_o, ov);
+          list.add(found, (uint32_t)v);
+          if (++since == full) {
+            since = 0;
+            __syncthreads();
+            if (__syncthreads_or(s_listed > KC_THREADS)) list.flush(a.off, qout_v, qout_e, qout_o, octr, &psc);
+          }
         }
+        list.flush(a.off, qout_v, qout_e, qout_o, octr, &psc);
       }
       ull out;
       if (!grid_sync_read(a.gs, a.err, a.timeout_ns, octr, &out)) return;
@@ -1092,7 +1144,7 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   uint32_t *qo0 = (uint32_t *)phde_buf(ctx, "kc.qo0", sizeof(uint32_t) * n);
   uint32_t *qo1 = (uint32_t *)phde_buf(ctx, "kc.qo1", sizeof(uint32_t) * n);
   ull *ctr = (ull *)phde_buf(ctx, "q.ctr", sizeof(ull) * 4);
-  const int64_t W = (n + 31) / 32;
+  const int64_t W = ((n + 31) / 32 + 3) & ~(int64_t)3;  // whole 16-byte pieces
   uint32_t *bms = (uint32_t *)phde_buf(ctx, "kc.bitmaps", sizeof(uint32_t) * 3 * W);
   if (!bms) return PHDE_ERR_OOM;
   PHDE_CK(ctx, cudaMemsetAsync(bms, 0, sizeof(uint32_t) * 3 * W, ctx->stream));
@@ -1111,8 +1163,10 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   // shared memory: the selection history, then (when it fits two blocks per SM) the frontier bitmap
   const size_t hist_bytes = sizeof(uint32_t) * (size_t)((P + 3) & ~3);
   const size_t bm_bytes = sizeof(uint32_t) * (size_t)W;
-  const int smem_bm = hist_bytes + bm_bytes <= 100 * 1024;
-  const size_t smem = hist_bytes + (smem_bm ? bm_bytes : 0);
+  // ... and the list of new vertices, 4096 entries, or 2048 beside the largest bitmaps
+  const int smem_bm = hist_bytes + bm_bytes <= 98 * 1024;
+  const int cap = smem_bm && hist_bytes + bm_bytes > 90 * 1024 ? 2 * KC_THREADS : 4 * KC_THREADS;
+  const size_t smem = hist_bytes + sizeof(uint32_t) * cap + (smem_bm ? bm_bytes : 0);
   PHDE_CK(ctx, cudaFuncSetAttribute(kcenters_bfs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kcenters_bfs_kernel, KC_THREADS, smem));
   if (per_sm < 1) return phde_fail(ctx, PHDE_ERR_CUDA, "kcenters kernel cannot be resident");
@@ -1148,6 +1202,7 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   a.bm[2] = bms + 2 * W;
   a.W = W;
   a.smem_bm = smem_bm;
+  a.cap = cap;
   a.edges = d_edges;
   // PHDE_BFS_TRACE=<file>: write the per-level timeline of this launch as CSV after it completes
   const char *trace_file = getenv("PHDE_BFS_TRACE");
