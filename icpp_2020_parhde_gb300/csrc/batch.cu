@@ -135,6 +135,7 @@ __global__ void __launch_bounds__(GT) batch_gram_kernel(Seg sg, const float *A, 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int b = sg.graph[s];
   const int nq = jcount ? jcount[4 * b] : nq_fixed;
+  const int rows = nq + (ones ? 1 : 0);  // Gram rows that are read
   const int64_t rb = sg.r0[s], re = sg.r1[s];
   float acc[8];
 #pragma unroll
@@ -166,6 +167,7 @@ __global__ void __launch_bounds__(GT) batch_gram_kernel(Seg sg, const float *A, 
     for (int t = 0; t < NX; t++) Xt[r2 + t * (GT / BB)][xi] = px[t];
     __syncthreads();
     if (r0 + RT < re) fetch(r0 + RT);
+    if (warp * 8 >= rows) continue;  // nothing but zero columns of A: 16.2 -> 9.5 ms over a layout's launches, 18.3M rows
 #pragma unroll 4
     for (int rr = 0; rr < RT; rr++) {
       const float x = Xt[rr][lane];
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(GT) batch_gram_kernel(Seg sg, const float *A, 
       acc[7] = fmaf(a1.w, x, acc[7]);
     }
   }
+  if (warp * 8 >= rows) return;  // no reader
   float *dst = part + ((int64_t)s * QCH + warp * 8) * BB + lane;
 #pragma unroll
   for (int m = 0; m < 8; m++) dst[m * BB] = acc[m];
@@ -244,33 +247,66 @@ __global__ void __launch_bounds__(bcgs_gs::NW * 32) batch_block_gs_kernel(const 
 }
 
 // S[v][j0_b + a] = sum_i X[v][i] R_b[i][a], a < nacc_b, with per-segment sums of deg * S^2 per column.
+// Tiles of FT rows: a thread takes a row and every fourth new column, then the FP64 sums go to one thread per (warp
+// slot, column) pair, packed -- a warp-wide FP64 instruction holds the pipe 16 clocks however many lanes it needs.
+// The sums run over rows w, w + 8, ... of the segment per slot w and then over the slots, as with a warp per row.
+// 18.3M rows, k = 10: 4.65 -> 2.88 ms.
+constexpr int FT = 64;
 __global__ void __launch_bounds__(GT) batch_form_kernel(Seg sg, const float *X, const float *Rall, const int *stall,
                                                         float *S, int lda, const double *deg, double *fpart) {
   __shared__ float Rs[BB][BB + 1];
+  __shared__ float Xs[FT][BB + 1], Vs[FT][BB + 1];
+  __shared__ double ds[FT];
   __shared__ double red[GT / 32][BB];
   const int s = blockIdx.x, b = sg.graph[s];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int tid = threadIdx.x, row = tid % FT, g = tid / FT;
   const int nacc = stall[4 * b + 3], j0 = stall[4 * b] - nacc;
-  for (int idx = threadIdx.x; idx < BB * BB; idx += GT) Rs[idx / BB][idx % BB] = Rall[(int64_t)b * BB * BB + idx];
-  __syncthreads();
+  for (int idx = tid; idx < BB * BB; idx += GT) Rs[idx / BB][idx % BB] = Rall[(int64_t)b * BB * BB + idx];
+  for (int idx = tid; idx < GT / 32 * BB; idx += GT) red[idx / BB][idx % BB] = 0.0;
+  const int64_t rb = sg.r0[s], re = sg.r1[s];
+  const bool sums = tid < 8 * nacc;
+  const int w = sums ? tid / nacc : 0, col = sums ? tid % nacc : 0;
   double dsum = 0;
   if (nacc > 0)
-    for (int64_t v = sg.r0[s] + warp; v < sg.r1[s]; v += nw) {
-      const float x = X[v * BB + lane];
-      float val = 0.f;
-#pragma unroll 8
-      for (int i = 0; i < BB; i++) val = fmaf(__shfl_sync(PHDE_FULL_MASK, x, i), Rs[i][lane], val);
-      if (lane < nacc) {
-        S[v * lda + j0 + lane] = val;
-        dsum += (double)val * (double)val * deg[v];
+    for (int64_t v0 = rb; v0 < re; v0 += FT) {
+      const int n = (int)(re - v0 < FT ? re - v0 : FT);
+      __syncthreads();
+      for (int idx = tid; idx < n * BB; idx += GT) Xs[idx / BB][idx % BB] = X[v0 * BB + idx];
+      if (tid < n) ds[tid] = deg[v0 + tid];
+      __syncthreads();
+      if (row < n) {
+        constexpr int NC = BB * FT / GT;
+        float val[NC];
+#pragma unroll
+        for (int t = 0; t < NC; t++) val[t] = 0.f;
+        for (int i = 0; i < BB; i++) {
+          const float x = Xs[row][i];
+#pragma unroll
+          for (int t = 0; t < NC; t++)
+            if (g + t * (GT / FT) < nacc) val[t] = fmaf(x, Rs[i][g + t * (GT / FT)], val[t]);
+        }
+#pragma unroll
+        for (int t = 0; t < NC; t++)
+          if (g + t * (GT / FT) < nacc) Vs[row][g + t * (GT / FT)] = val[t];
       }
+      __syncthreads();
+      for (int idx = tid; idx < n * nacc; idx += GT) {
+        const int r = idx / nacc, a = idx - r * nacc;
+        S[(v0 + r) * lda + j0 + a] = Vs[r][a];
+      }
+      if (sums)
+        for (int r = w; r < n; r += 8) {
+          const double v = (double)Vs[r][col];
+          dsum = fma(__dmul_rn(v, v), ds[r], dsum);
+        }
     }
-  red[warp][lane] = dsum;
   __syncthreads();
-  if (warp == 0) {
+  if (sums) red[w][col] = dsum;
+  __syncthreads();
+  if (tid < BB) {
     double t = 0;
-    for (int w = 0; w < nw; w++) t += red[w][lane];
-    fpart[(int64_t)s * BB + lane] = t;
+    for (int q = 0; q < GT / 32; q++) t += red[q][tid];
+    fpart[(int64_t)s * BB + tid] = t;
   }
 }
 
@@ -285,43 +321,58 @@ __global__ void batch_dd_kernel(Seg sg, const double *fpart, const int *stall, i
 }
 
 // Coordinates of a segment's rows: X_b = S_b Y_b (FP32 products and row sums), written column-major per
-// graph at out + c * vbase[b]; per-segment sums of squares per coordinate.
+// graph at out + c * vbase[b]; per-segment sums of squares per coordinate.  A thread per row of a staged tile adds
+// its row's products in the order of a 32-lane shuffle tree (a warp per row with that tree was 4.5 ms on 18.3M rows,
+// k = 10, five shuffles a coordinate and ten lanes of 32 in use; 0.74 ms now); the squares go to one thread per
+// (row mod 8, coordinate), summed as with eight warps.
+template <int KB>
+__device__ __forceinline__ float tree_row_sum(const float *row, const float *Ys, int k, int c, int t) {
+  float a[KB];
+#pragma unroll
+  for (int q = 0; q < KB; q++) a[q] = q < k ? __fmul_rn(row[q], Ys[q * c + t]) : 0.f;
+#pragma unroll
+  for (int o = KB / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int q = 0; q < o; q++) a[q] = __fadd_rn(a[q], a[q + o]);
+  return a[0];
+}
+
 __global__ void __launch_bounds__(GT) batch_coords_kernel(Seg sg, const float *S, int k, const double *Yall, int c,
                                                           const int64_t *vbase, double *out, double *cpart) {
   __shared__ float Ys[BB * MAXC];
+  __shared__ float rows[GT * (BB + 1)];
+  __shared__ float xs[MAXC][GT];
   __shared__ double red[GT / 32][MAXC];
   const int s = blockIdx.x, b = sg.graph[s];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int tid = threadIdx.x, ld = k | 1;
   const double *Y = Yall + (int64_t)b * k * c;  // column-major k x c
-  for (int idx = threadIdx.x; idx < k * c; idx += GT) Ys[(idx % k) * c + idx / k] = (float)Y[idx];
-  __syncthreads();
+  for (int idx = tid; idx < k * c; idx += GT) Ys[(idx % k) * c + idx / k] = (float)Y[idx];
   const int64_t vb = vbase[b], nb = vbase[b + 1] - vb;
-  double ss[MAXC] = {0, 0, 0, 0};
-  for (int64_t v = sg.r0[s] + warp; v < sg.r1[s]; v += nw) {
-    float acc[MAXC] = {0.f, 0.f, 0.f, 0.f};
-    if (lane < k) {
-      const float sv = S[v * k + lane];
-#pragma unroll
-      for (int t = 0; t < MAXC; t++)
-        if (t < c) acc[t] = sv * Ys[lane * c + t];
-    }
-#pragma unroll
-    for (int t = 0; t < MAXC; t++) {
-      if (t >= c) break;
-      const float x = warp_sum(acc[t]);
-      if (lane == 0) {
-        out[c * vb + (int64_t)t * nb + (v - vb)] = (double)x;
-        ss[t] = fma((double)x, (double)x, ss[t]);
+  const int w = tid & 7, t0 = tid >> 3;  // the sum this thread keeps, below 8 * c
+  double ss = 0;
+  for (int64_t v0 = sg.r0[s]; v0 < sg.r1[s]; v0 += GT) {
+    const int n = (int)(sg.r1[s] - v0 < GT ? sg.r1[s] - v0 : GT);
+    __syncthreads();
+    for (int idx = tid; idx < n * k; idx += GT) rows[(idx / k) * ld + idx % k] = S[v0 * k + idx];
+    __syncthreads();
+    if (tid < n)
+      for (int t = 0; t < c; t++) {
+        const float x = k <= 16 ? tree_row_sum<16>(rows + tid * ld, Ys, k, c, t)
+                                : tree_row_sum<32>(rows + tid * ld, Ys, k, c, t);
+        out[c * vb + (int64_t)t * nb + (v0 + tid - vb)] = (double)x;
+        xs[t][tid] = x;
       }
-    }
+    __syncthreads();
+    if (t0 < c)
+      for (int r = w; r < n; r += 8) ss = fma((double)xs[t0][r], (double)xs[t0][r], ss);
   }
-  if (lane == 0)
-    for (int t = 0; t < MAXC; t++) red[warp][t] = ss[t];
+  if (t0 < c) red[w][t0] = ss;
   __syncthreads();
-  if (threadIdx.x < MAXC) {
+  if (tid < MAXC) {
     double t = 0;
-    for (int w = 0; w < nw; w++) t += red[w][threadIdx.x];
-    cpart[(int64_t)s * MAXC + threadIdx.x] = t;
+    if (tid < c)
+      for (int q = 0; q < GT / 32; q++) t += red[q][tid];
+    cpart[(int64_t)s * MAXC + tid] = t;
   }
 }
 
