@@ -34,8 +34,8 @@
 
 namespace {
 
-constexpr int RT = 2048;          // CSR entries per raster tile
-constexpr int RT_THREADS = 512;   // threads per raster CTA
+constexpr int RT = 1024;          // CSR entries per raster tile
+constexpr int RT_THREADS = 256;   // threads per raster CTA
 constexpr int RCHUNK = 32;        // pixels per raster chunk
 constexpr int RGROUP = 8;         // pixels whose owner reads a thread issues together
 constexpr int SEL_THREADS = 1024; // the cut-selection CTA
@@ -129,22 +129,64 @@ __global__ void draw_scale_kernel(const double *x, const double *y, int64_t n, d
   }
 }
 
-// Row of every CSR entry, one warp per vertex.
-__global__ void draw_rows_kernel(const int64_t *off, int64_t n, uint32_t *erow) {
+// Row of every CSR entry, one warp per vertex; *unsorted is set when a row's neighbours are not in increasing order.
+__global__ void draw_rows_kernel(const int64_t *off, const uint32_t *adj, int64_t n, uint32_t *erow, int *unsorted) {
   const int lane = threadIdx.x & 31;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < n; u += nw) {
     const int64_t e1 = off[u + 1];
-    for (int64_t e = off[u] + lane; e < e1; e += 32) erow[e] = (uint32_t)u;
+    const int64_t e0 = off[u];
+    bool bad = false;
+    for (int64_t e = e0 + lane; e < e1; e += 32) {
+      erow[e] = (uint32_t)u;
+      bad |= e > e0 && adj[e] < adj[e - 1];
+    }
+    if (bad) *unsorted = 1;
   }
 }
 
-// length(floor(u), floor(v)) of draw_graph.c:130-133 as float: the squared length is an exact integer below
-// 2^53 for images below 2^26 pixels a side, so only the square root and the float conversion round.
-__device__ __forceinline__ float entry_length(int2 p, int2 q) {
-  const double dx = (double)(q.x - p.x), dy = (double)(q.y - p.y);
-  return __double2float_rn(__dsqrt_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy))));
+// Bit e: entry e = (u, v) has u < v and the graph has an entry (v, u) -- a later one, as rows are in order -- which
+// draws the same line back (draw_raster_kernel).  Found by binary search; no bits for a CSR with unsorted rows.
+__global__ void draw_mirror_kernel(const int64_t *off, const uint32_t *adj, const uint32_t *erow, int64_t nnz,
+                                   const int *unsorted, uint32_t *mirror) {
+  const bool usable = *unsorted == 0;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t e0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); e0 < nnz; e0 += stride) {
+    const int64_t e = e0 + (threadIdx.x & 31);
+    bool found = false;
+    if (usable && e < nnz) {
+      const uint32_t u = erow[e], v = adj[e];
+      if (u < v) {
+        int64_t lo = off[v], hi = off[v + 1];  // first entry >= u
+        while (lo < hi) {
+          const int64_t mid = (lo + hi) >> 1;
+          if (__ldg(adj + mid) < u)
+            lo = mid + 1;
+          else
+            hi = mid;
+        }
+        found = lo < off[v + 1] && __ldg(adj + lo) == u;
+      }
+    }
+    const uint32_t word = __ballot_sync(PHDE_FULL_MASK, found);
+    if ((threadIdx.x & 31) == 0) mirror[e0 >> 5] = word;
+  }
 }
+
+// length(floor(u), floor(v)) of draw_graph.c:130-133 as float, from the squared length, an exact integer (images are
+// below 2^20 pixels a side): only the square root and the float conversion round.  Below 2^24 the FP32 square root
+// gives the same bits: rounding to double first would have to land on the midpoint z of two floats, and an integer
+// other than z^2 is further from it (2^(2a-48) for z in [2^a, 2^(a+1))) than a double's half unit reaches
+// (2^(2a-50)).  FP64 square roots of every entry were about a fifth of the rasteriser's time.
+__device__ __forceinline__ ull entry_length2(int2 p, int2 q) {
+  const long long dx = q.x - p.x, dy = q.y - p.y;
+  return (ull)(dx * dx + dy * dy);
+}
+__device__ __forceinline__ float length_of(ull d2) {
+  if (d2 < (1ull << 24)) return __fsqrt_rn((float)(uint32_t)d2);
+  return __double2float_rn(__dsqrt_rn((double)d2));
+}
+__device__ __forceinline__ float entry_length(int2 p, int2 q) { return length_of(entry_length2(p, q)); }
 
 // bin = (int) floor((len / max) * 7) in float (draw_graph.c:323); 0 / 0 (every entry of length 0) is not a
 // number, whose conversion gives INT_MIN on x86-64, a bin no case names: drawn black like bin 7.
@@ -154,15 +196,16 @@ __device__ __forceinline__ int entry_bin(float len, float mx) {
   return (int)floorf(q);
 }
 
+// Largest squared length (the length grows with it).
 __global__ void draw_maxlen_kernel(const uint32_t *erow, const uint32_t *adj, const int2 *pix, int64_t nnz,
-                                   unsigned *maxbits) {
-  float mx = 0.f;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += (int64_t)gridDim.x * blockDim.x)
-    mx = fmaxf(mx, entry_length(pix[erow[e]], pix[adj[e]]));
-  // non-negative floats order like their bit patterns
-  unsigned b = __float_as_uint(mx);
-  b = __reduce_max_sync(PHDE_FULL_MASK, b);
-  if ((threadIdx.x & 31) == 0 && b) atomicMax(maxbits, b);
+                                   ull *max2) {
+  ull mx = 0;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += (int64_t)gridDim.x * blockDim.x) {
+    const ull d2 = entry_length2(pix[erow[e]], pix[adj[e]]);
+    mx = d2 > mx ? d2 : mx;
+  }
+  mx = warp_max_u64(mx);
+  if ((threadIdx.x & 31) == 0 && mx) atomicMax(max2, mx);
 }
 
 // The Bresenham state of one line at major step k.
@@ -173,7 +216,8 @@ struct Line {
   uint32_t M, m, r;  // major and minor extents, remainder of (k m + M - floor(M/2) - 1) mod M
 };
 
-__device__ __forceinline__ void line_at(Line &L, int2 p, int2 q, uint32_t k) {
+// The line from p to q at its first pixel: no division.
+__device__ __forceinline__ void line_start(Line &L, int2 p, int2 q) {
   const int dx = q.x - p.x, dy = q.y - p.y;
   const uint32_t adx = (uint32_t)abs(dx), ady = (uint32_t)abs(dy);
   const int sx = p.x < q.x ? 1 : -1, sy = p.y < q.y ? 1 : -1;
@@ -184,15 +228,27 @@ __device__ __forceinline__ void line_at(Line &L, int2 p, int2 q, uint32_t k) {
   L.smaj_y = xmajor ? 0 : sy;
   L.smin_x = xmajor ? 0 : sx;
   L.smin_y = xmajor ? sy : 0;
-  uint32_t kk = 0;
-  L.r = 0;
-  if (L.M > 0) {
-    const ull num = (ull)k * L.m + (L.M - L.M / 2u - 1u);
+  L.r = L.M > 0 ? L.M - L.M / 2u - 1u : 0u;
+  L.cx = p.x;
+  L.cy = p.y;
+}
+
+// ... and at major step k; the products stay below 2^32 for extents below 2^16.
+__device__ __forceinline__ void line_at(Line &L, int2 p, int2 q, uint32_t k) {
+  line_start(L, p, q);
+  if (k == 0) return;  // k <= M, so M > 0 from here on
+  uint32_t kk;
+  if (L.M < 65536u) {
+    const uint32_t num = k * L.m + L.r;
+    kk = num / L.M;
+    L.r = num - kk * L.M;
+  } else {
+    const ull num = (ull)k * L.m + L.r;
     kk = (uint32_t)(num / L.M);
     L.r = (uint32_t)(num % L.M);
   }
-  L.cx = p.x + L.smaj_x * (int)k + L.smin_x * (int)kk;
-  L.cy = p.y + L.smaj_y * (int)k + L.smin_y * (int)kk;
+  L.cx += L.smaj_x * (int)k + L.smin_x * (int)kk;
+  L.cy += L.smaj_y * (int)k + L.smin_y * (int)kk;
 }
 
 __device__ __forceinline__ void line_step(Line &L) {
@@ -206,14 +262,30 @@ __device__ __forceinline__ void line_step(Line &L) {
   }
 }
 
+__device__ __forceinline__ uint32_t gcd_u32(uint32_t a, uint32_t b) {
+  while (b) {
+    const uint32_t t = a % b;
+    a = b;
+    b = t;
+  }
+  return a;
+}
+
 // One CTA per tile of RT entries: bins and per-tile counts of bins 0, 1, 5, 6 (tcnt[tile * 4 + j]), then
 // every pixel of the tile's lines.  SKIP: tiles run from the last to the first, and a pixel whose owner (read
 // through L1, possibly stale) is already a later entry needs no atomic -- owners only grow, so a stale value
 // that is already larger is still larger.
+// An entry with its mirror bit set is drawn back by a later entry, which owns every pixel the two share.  After k
+// major steps of M, with minor extent m, the line there is at minor floor((k m + c) / M), c = M - floor(M/2) - 1, and
+// the line back at ceil((k m - c) / M): they differ where k m mod M = M / 2 exactly, M even -- with g = gcd(M, m) at
+// k = (t + 1/2) M / g, t < g, when M / g is even, and nowhere else.  Only those pixels (mostly none or one) are
+// drawn; the reported pixel writes count the whole line.  R-MAT 18 at
+// 4172 x 4172: 1.63 -> 1.34 ms, 1.23 with no division at a line's start, 1.14 with tiles of 1024 entries and 256 threads
+// (2048 and 512: 1.23; the tiles' ends wait for their longest lines).  75 -> 72 instructions a drawn pixel are left.
 template <bool SKIP>
 __global__ void __launch_bounds__(RT_THREADS) draw_raster_kernel(const uint32_t *erow, const uint32_t *adj,
-                                                                 const int2 *pix, int64_t nnz,
-                                                                 const unsigned *maxbits, unsigned W, unsigned H,
+                                                                 const int2 *pix, int64_t nnz, const uint32_t *mirror,
+                                                                 const ull *max2, unsigned W, unsigned H,
                                                                  uint32_t *owner, uint8_t *bin, uint32_t *tcnt,
                                                                  ull *pixels) {
   __shared__ int2 s_a[RT], s_b[RT];
@@ -224,9 +296,10 @@ __global__ void __launch_bounds__(RT_THREADS) draw_raster_kernel(const uint32_t 
   const int64_t tile = SKIP ? (int64_t)gridDim.x - 1 - blockIdx.x : (int64_t)blockIdx.x;
   const int64_t e0 = tile * RT;
   const int cnt = (int)min((int64_t)RT, nnz - e0);
-  const float mx = __uint_as_float(*maxbits);
+  const float mx = length_of(*max2);
+  const unsigned tiles_w = (W + 7) >> 3;
   if (tid < 4) s_cnt[tid] = 0;
-  uint32_t c0 = 0, c1 = 0, c5 = 0, c6 = 0;
+  uint32_t c0 = 0, c1 = 0, c5 = 0, c6 = 0, whole = 0;  // whole: pixels of the lines, drawn here or not
   for (int i = tid; i < RT; i += RT_THREADS) {
     uint32_t len = 0;
     if (i < cnt) {
@@ -235,6 +308,19 @@ __global__ void __launch_bounds__(RT_THREADS) draw_raster_kernel(const uint32_t 
       s_a[i] = p;
       s_b[i] = q;
       len = (uint32_t)max(abs(q.x - p.x), abs(q.y - p.y)) + 1u;
+      whole += len;
+      if ((mirror[e >> 5] >> (e & 31)) & 1u) {
+        const uint32_t M = len - 1u, m = (uint32_t)min(abs(q.x - p.x), abs(q.y - p.y));
+        len = 0;
+        if (m > 0 && __ffs(M) > __ffs(m)) {  // M / g even: more factors of two in M than in m
+          const uint32_t step = M / gcd_u32(M, m);
+          for (uint32_t k = step / 2; k < M; k += step) {
+            Line L;
+            line_at(L, p, q, k);
+            atomicMax(&owner[tile_index((unsigned)L.cx, (unsigned)L.cy, tiles_w)], (uint32_t)(e + 1));
+          }
+        }
+      }
       const int b = entry_bin(entry_length(p, q), mx);
       bin[e] = (uint8_t)b;
       c0 += b == 0;
@@ -248,6 +334,8 @@ __global__ void __launch_bounds__(RT_THREADS) draw_raster_kernel(const uint32_t 
   c1 = __reduce_add_sync(PHDE_FULL_MASK, c1);
   c5 = __reduce_add_sync(PHDE_FULL_MASK, c5);
   c6 = __reduce_add_sync(PHDE_FULL_MASK, c6);
+  whole = __reduce_add_sync(PHDE_FULL_MASK, whole);
+  if (lane == 0) atomicAdd(pixels, (ull)whole);
   __syncthreads();
   if (lane == 0) {
     atomicAdd(&s_cnt[0], c0);
@@ -291,9 +379,7 @@ __global__ void __launch_bounds__(RT_THREADS) draw_raster_kernel(const uint32_t 
   __syncthreads();
   if (tid < 4) tcnt[tile * 4 + tid] = s_cnt[tid];
   const uint32_t P = s_pre[RT];
-  if (tid == 0) atomicAdd(pixels, (ull)P);
   const uint32_t nch = (P + RCHUNK - 1) / RCHUNK;
-  const unsigned tiles_w = (W + 7) >> 3;
   for (uint32_t c = tid; c < nch; c += RT_THREADS) {
     const uint32_t p0 = c * RCHUNK, pend = min(p0 + RCHUNK, P);
     int lo = 0, hi = cnt;  // s_pre[lo] <= p0 < s_pre[hi]
@@ -315,18 +401,19 @@ __global__ void __launch_bounds__(RT_THREADS) draw_raster_kernel(const uint32_t 
       uint32_t tg[RGROUP];
 #pragma unroll
       for (int q = 0; q < RGROUP; q++) {
-        tg[q] = 0;  // 0: no pixel (past the chunk, or outside the image)
+        tg[q] = 0;  // 0: past the chunk
         if (p + q < pend) {
-          if ((unsigned)L.cx < W && (unsigned)L.cy < H) {
-            at[q] = tile_index((unsigned)L.cx, (unsigned)L.cy, tiles_w);
-            tg[q] = tag;
-          }
+          // inside the image: between the line's ends, which draw_scale_kernel clamps to it
+          at[q] = tile_index((unsigned)L.cx, (unsigned)L.cy, tiles_w);
+          tg[q] = tag;
           if (--left == 0) {
             if (p + q + 1 < pend) {
-              i++;
-              left = s_pre[i + 1] - s_pre[i];
-              line_at(L, s_a[i], s_b[i], 0);
-              tag++;
+              do {  // the next line with pixels
+                i++;
+                tag++;
+                left = s_pre[i + 1] - s_pre[i];
+              } while (left == 0);
+              line_start(L, s_a[i], s_b[i]);
             }
           } else {
             line_step(L);
@@ -604,13 +691,20 @@ extern "C" int phde_draw(phde_ctx *ctx, const double *x, const double *y, phde_d
   uint32_t *tcnt = (uint32_t *)phde_buf(ctx, "draw.tcnt", sizeof(uint32_t) * 4 * std::max<int64_t>(ntiles, 1));
   ull *misc = (ull *)phde_buf(ctx, "draw.misc", sizeof(ull) * 8);
   if (!owner || !packed || !erow || !bin || !tcnt || !misc) return PHDE_ERR_OOM;
-  unsigned *maxbits = (unsigned *)misc;        // misc[0] low word
+  ull *max2 = misc;                            // largest squared length
   ull *pixels = misc + 1;
   int64_t *cuts = (int64_t *)(misc + 2);       // misc[2..5]
   cudaEventRecord(ctx->ev[2], ctx->stream);
+  uint32_t *mirror = (uint32_t *)phde_buf(ctx, "draw.mirror", sizeof(uint32_t) * std::max<int64_t>((nnz + 31) / 32, 1));
+  if (!mirror) return PHDE_ERR_OOM;
   if (ctx->draw_rows_epoch != ctx->graph_epoch || ctx->draw_rows_buf != (void *)erow) {
     if (nnz > 0) {
-      draw_rows_kernel<<<grid_of(ctx, n * 32, 256), 256, 0, ctx->stream>>>(ctx->d_off, n, erow);
+      int *unsorted = (int *)(misc + 7);
+      PHDE_CK(ctx, cudaMemsetAsync(unsorted, 0, sizeof(int), ctx->stream));
+      draw_rows_kernel<<<grid_of(ctx, n * 32, 256), 256, 0, ctx->stream>>>(ctx->d_off, ctx->d_adj, n, erow, unsorted);
+      PHDE_LAUNCHED(ctx);
+      draw_mirror_kernel<<<grid_of(ctx, nnz, 256), 256, 0, ctx->stream>>>(ctx->d_off, ctx->d_adj, erow, nnz, unsorted,
+                                                                          mirror);
       PHDE_LAUNCHED(ctx);
     }
     ctx->draw_rows_epoch = ctx->graph_epoch;
@@ -621,15 +715,15 @@ extern "C" int phde_draw(phde_ctx *ctx, const double *x, const double *y, phde_d
   PHDE_CK(ctx, cudaMemsetAsync(misc, 0, sizeof(ull) * 8, ctx->stream));
   PHDE_CK(ctx, cudaMemsetAsync(owner, 0, sizeof(uint32_t) * npix_tiled, ctx->stream));
   if (nnz > 0) {
-    draw_maxlen_kernel<<<grid_of(ctx, nnz, 256), 256, 0, ctx->stream>>>(erow, ctx->d_adj, pix, nnz, maxbits);
+    draw_maxlen_kernel<<<grid_of(ctx, nnz, 256), 256, 0, ctx->stream>>>(erow, ctx->d_adj, pix, nnz, max2);
     PHDE_LAUNCHED(ctx);
     cudaEventRecord(ctx->ev[3], ctx->stream);
     const char *rv = getenv("PHDE_DRAW_RASTER");
     if (rv && strcmp(rv, "plain") == 0)
-      draw_raster_kernel<false><<<(unsigned)ntiles, RT_THREADS, 0, ctx->stream>>>(erow, ctx->d_adj, pix, nnz, maxbits,
+      draw_raster_kernel<false><<<(unsigned)ntiles, RT_THREADS, 0, ctx->stream>>>(erow, ctx->d_adj, pix, nnz, mirror, max2,
                                                                                   W, H, owner, bin, tcnt, pixels);
     else
-      draw_raster_kernel<true><<<(unsigned)ntiles, RT_THREADS, 0, ctx->stream>>>(erow, ctx->d_adj, pix, nnz, maxbits,
+      draw_raster_kernel<true><<<(unsigned)ntiles, RT_THREADS, 0, ctx->stream>>>(erow, ctx->d_adj, pix, nnz, mirror, max2,
                                                                                  W, H, owner, bin, tcnt, pixels);
     PHDE_LAUNCHED(ctx);
     cudaEventRecord(ctx->ev[4], ctx->stream);
@@ -661,8 +755,7 @@ extern "C" int phde_draw(phde_ctx *ctx, const double *x, const double *y, phde_d
     info->ymin = ymin;
     info->ymax = ymax;
     info->aspect = aspect;
-    unsigned mb = (unsigned)(hm[0] & 0xffffffffu);
-    memcpy(&info->max_edge_length, &mb, sizeof(float));
+    info->max_edge_length = (float)std::sqrt((double)hm[0]);
     info->pixels = (int64_t)hm[1];
     float t01 = 0, t25 = 0, t34 = 0;
     cudaEventElapsedTime(&t01, ctx->ev[0], ctx->ev[1]);

@@ -162,3 +162,43 @@ def test_draw_plain_raster_variant_matches(monkeypatch):
     with Context(0) as ctx:
         img, _ = gpu_image(ctx, g, x, y)
     assert np.array_equal(img, pngdecode.read(png))
+
+
+@pytest.mark.parametrize("case", ["symmetric", "one_way", "unsorted", "duplicates", "half_slopes"])
+def test_draw_entries_and_their_mirrors(gpu_ctx, case):
+    """An entry that a later one draws back is drawn only where the two lines differ: against the oracle with every
+    mirror present, with some missing, with unsorted rows (no mirrors are used), with parallel entries and loops, and
+    on an integer lattice full of the slopes where the two directions differ."""
+    rng = np.random.default_rng(31)
+    n = 400
+    x, y = _random_positions(n, 32, (40.0, 40.0))
+    u, v = rng.integers(0, n, 3000), rng.integers(0, n, 3000)
+    if case == "half_slopes":
+        side = 20
+        n = side * side
+        x, y = (np.arange(n) % side).astype(float), (np.arange(n) // side).astype(float)
+        u = rng.integers(0, n, 3000)
+        d = rng.choice([1, 2 * side + 1, side + 2, 4 * side + 2, 6 * side + 2, 3 * side], 3000)
+        v = (u + d) % n
+    s, t = np.concatenate([u, v]), np.concatenate([v, u])
+    if case == "one_way":
+        keep = rng.random(s.size) < 0.6
+        s, t = s[keep], t[keep]
+    if case != "duplicates":
+        key = np.unique(s * n + t)
+        s, t = key // n, key % n
+    if case == "unsorted":
+        p = rng.permutation(s.size)
+        s, t = s[p], t[p]
+        o = np.argsort(s, kind="stable")
+        s, t = s[o], t[o]
+    else:
+        o = np.argsort(s * n + t, kind="stable")
+        s, t = s[o], t[o]
+    off = np.zeros(n + 1, dtype=np.uint32)
+    off[1:] = np.cumsum(np.bincount(s, minlength=n))
+    g = graphs.CSRGraph(off, t.astype(np.uint32))
+    img, info = gpu_image(gpu_ctx, g, x, y)
+    ref, ml = orc.draw(g, x, y)
+    assert img.shape == ref.shape and np.array_equal(img, ref)
+    assert info["max_edge_length"] == np.float32(ml)
