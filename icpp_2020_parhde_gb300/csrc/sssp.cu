@@ -292,15 +292,18 @@ __global__ void __launch_bounds__(SS_THREADS, MINB) sssp_nearfar_kernel(SsArgs a
 // ---- graphs of bounded degree (grids, meshes, geometric graphs): a lane group per frontier vertex ----
 // A round is a chain of dependent memory trips ended by a grid barrier, whatever it relaxes; the edge-balanced
 // kernel above spends about a third of its trips finding the owner of every edge.  Where no row is longer than
-// SG_LANES * 4, eight lanes take one frontier entry (vertex, row start and length in one 16-byte word) and R edges
-// each, all R in flight: entry -> adjacency, weight and the vertex's distance -> the neighbours' distances -> the
+// SG_MAX_ROW, G lanes take one frontier entry (vertex, row start and length in one 16-byte word) and R edges each:
+// entry -> adjacency, weight and the vertex's distance -> the neighbours' distances -> the
 // updates -> push.  The update is a reduction (no value returned) with the duplicate stamp's exchange beside it
 // instead of after it: a thread that found the neighbour's distance larger pushes when its stamp is the round's
 // first, whether its own minimum was the one that stayed -- some thread lowered the distance in this round, and
 // every thread that did so takes the stamp.  Bands, far pile and results as in sssp_nearfar_kernel.
 // Measured, 20 passes: 256^3 grid 238 -> 180 ms (12.4 -> 9.4 us a round), 65 x 61 x 70 grid 24.8 -> 20.4 ms (6.8 ->
 // 5.6 us a round; 4.7 us of a round is the chain itself, measured with a band that leaves 7k edges a round).
-constexpr int SG_LANES = 8;
+// Shapes (G, R), passes of a layout with k = 10: rows up to 16, 300k vertices (16, 1) 94 ms, (8, 2) 101; rows up to 32,
+// 300k vertices (16, 2) 42, (32, 1) 44, (8, 4) 54; 2M vertices in 3-D 33, 40 and 36.  Fewer lanes with more edges each
+// lose on grids too: 256^3 (8, 1) 233, (4, 2) 255, (2, 4) 319 ms a layout.
+constexpr int SG_MAX_ROW = 32;
 
 struct PushRScratch {
   uint32_t warp_tot[32];
@@ -346,11 +349,11 @@ __device__ __forceinline__ void block_push_r(unsigned nearm, unsigned farm, cons
   }
 }
 
-template <int R, int MINB>
+template <int G, int R, int MINB>
 __global__ void __launch_bounds__(SS_THREADS, MINB) sssp_group_kernel(SsArgs a) {
   __shared__ PushRScratch psc;
   __shared__ ull red[32];
-  const int tid = threadIdx.x, gl = tid & (SG_LANES - 1);
+  const int tid = threadIdx.x, gl = tid & (G - 1);
   const int64_t gstride = (int64_t)gridDim.x * blockDim.x;
   const int64_t gbase = (int64_t)blockIdx.x * blockDim.x;
   const int64_t src = *a.src;
@@ -375,17 +378,17 @@ __global__ void __launch_bounds__(SS_THREADS, MINB) sssp_group_kernel(SsArgs a) 
       uint32_t *far_in = (phase & 1) ? a.far1 : a.far0;
       unsigned *fctr = a.farctr + (phase & 1);
       if (blockIdx.x == 0 && tid == 0) ctr[(step + 1) & 3] = 0u;
-      const int64_t lanes = (int64_t)f_cnt * SG_LANES;
+      const int64_t lanes = (int64_t)f_cnt * G;
       for (int64_t base = gbase; base < lanes; base += gstride) {
         uint32_t v[R], ov[R], dv[R];
         unsigned nearm = 0, farm = 0;
         if (base + tid < lanes) {
-          const uint4 en = __ldcg(qin + (base + tid) / SG_LANES);
+          const uint4 en = __ldcg(qin + (base + tid) / G);
           const int32_t du = __ldcg(a.dist + en.x);
           int32_t nd[R], old[R];
 #pragma unroll
           for (int r = 0; r < R; r++) {
-            const uint32_t e = gl + r * SG_LANES;
+            const uint32_t e = gl + r * G;
             const bool has = e < en.z;
             v[r] = has ? __ldg(a.adj + en.y + e) : en.x;  // the vertex itself: never an improvement
             nd[r] = has ? __ldg(a.w + en.y + e) : 0;
@@ -591,7 +594,7 @@ int phde_run_sssp(phde_ctx *ctx, const int64_t *d_src, int32_t *d_col, int32_t d
   if (delta < 1) delta = 1;
   const char *le = getenv("PHDE_SSSP_LOCAL");
   const int lmax = le ? std::max(0, atoi(le)) : 0;
-  const bool group = lmax == 0 && ctx->w_maxdeg <= 4 * SG_LANES;
+  const bool group = lmax == 0 && ctx->w_maxdeg <= SG_MAX_ROW;
   uint32_t *qv0, *qv1, *qe0 = nullptr, *qe1 = nullptr, *qo0 = nullptr, *qo1 = nullptr;
   if (group) {
     qv0 = (uint32_t *)phde_buf(ctx, "ss.q0", sizeof(uint4) * n);
@@ -622,19 +625,22 @@ int phde_run_sssp(phde_ctx *ctx, const int64_t *d_src, int32_t *d_col, int32_t d
   PHDE_CK(ctx, cudaMemsetAsync(farctr, 0, sizeof(unsigned) * 2, ctx->stream));
   PHDE_CK(ctx, cudaMemsetAsync(minfar, 0xff, sizeof(ull) * 2, ctx->stream));
   if ((rc = phde_reset_sync(ctx))) return rc;
-  // Resident CTAs per SM: one (with the registers it wants) below 2^20 vertices, where rounds are short and
-  // latency-bound (65 x 61 x 70 grid, lane groups: 20.4 ms for 20 passes against 21.0 with two), two (registers
-  // capped at 32) on larger graphs (256^3 grid: 180 ms against 218 with one); PHDE_SSSP_CTAS=1 or 2 picks outright.
+  // Resident CTAs per SM: one (with the registers it wants) on small graphs, whose rounds are short, two (registers
+  // capped at 32) on larger ones; PHDE_SSSP_CTAS=1 or 2 picks outright.  Lane groups change over at 2^18 vertices
+  // (65 x 61 x 70 grid, layout: 23.7 ms with two, 24.6 with one; 300k-vertex geometric graph of degree 8: 44 against
+  // 49), the edge-balanced kernel at 2^20 (64^3 grid: 1.5 ms per pass with one against 2.1; 256^3: 14.3 with two
+  // against 16.1).
   const char *ce = getenv("PHDE_SSSP_CTAS");
-  const int want = ce ? (atoi(ce) == 1 ? 1 : 2) : (n < ((int64_t)1 << 20) ? 1 : 2);
-  const int R = ctx->w_maxdeg <= SG_LANES ? 1 : ctx->w_maxdeg <= 2 * SG_LANES ? 2 : 4;
+  const int want = ce ? (atoi(ce) == 1 ? 1 : 2) : (n < ((int64_t)1 << (group ? 18 : 20)) ? 1 : 2);
   const void *kfn = want == 1 ? (const void *)sssp_nearfar_kernel<1> : (const void *)sssp_nearfar_kernel<2>;
-  if (group && want == 1)
-    kfn = R == 1 ? (const void *)sssp_group_kernel<1, 1> : R == 2 ? (const void *)sssp_group_kernel<2, 1>
-                                                                  : (const void *)sssp_group_kernel<4, 1>;
-  else if (group)
-    kfn = R == 1 ? (const void *)sssp_group_kernel<1, 2> : R == 2 ? (const void *)sssp_group_kernel<2, 2>
-                                                                  : (const void *)sssp_group_kernel<4, 2>;
+  if (group) {  // (lanes, edges per lane) by the longest row
+    const int shape = ctx->w_maxdeg <= 8 ? 0 : ctx->w_maxdeg <= 16 ? 1 : 2;
+    static const void *const kernels[3][2] = {
+        {(const void *)sssp_group_kernel<8, 1, 1>, (const void *)sssp_group_kernel<8, 1, 2>},
+        {(const void *)sssp_group_kernel<16, 1, 1>, (const void *)sssp_group_kernel<16, 1, 2>},
+        {(const void *)sssp_group_kernel<16, 2, 1>, (const void *)sssp_group_kernel<16, 2, 2>}};
+    kfn = kernels[shape][want - 1];
+  }
   // block-local rounds per grid round (PHDE_SSSP_LOCAL, none by default): each block keeps relaxing the
   // vertices it improved below the band limit (up to SS_LQ of them) this many times before the grid
   // barrier.  On a 256^3 grid four local rounds took 10-12.5 ms per pass on some runs and 43-50 ms on

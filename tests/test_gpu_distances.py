@@ -243,15 +243,15 @@ def test_cluster_kcenters_duplicate_sources_and_fixed_sources(gpu_ctx):
 
 @pytest.mark.parametrize("make", [
     lambda: graphs.path_graph(700),
-    lambda: graphs.mesh(60, 41, seed=21),                             # at most 8 neighbours: one edge per lane
-    lambda: graphs.rgg(9000, dim=2, avg_degree=5, seed=22),           # up to 16: two
-    lambda: graphs.rgg(20000, dim=2, avg_degree=9, seed=23),          # up to 32: four
+    lambda: graphs.mesh(60, 41, seed=21),                             # at most 8 neighbours: eight lanes
+    lambda: graphs.rgg(9000, dim=2, avg_degree=5, seed=22),           # up to 16: sixteen lanes
+    lambda: graphs.rgg(20000, dim=2, avg_degree=9, seed=23),          # up to 32: two edges per lane
     lambda: _two_stars(31, 5),                                        # rows of exactly 32
     lambda: _two_stars(32, 5),                                        # 33: the edge-balanced kernel
 ], ids=["path700", "mesh60x41", "rgg5", "rgg9", "deg32", "deg33"])
 @pytest.mark.parametrize("ctas,delta", [("1", None), ("2", "100")])
 def test_sssp_lane_groups_exact(gpu_ctx, monkeypatch, make, ctas, delta):
-    """The lane-group kernel at every number of edges per lane, with the wide band and with many bands."""
+    """The lane-group kernel in each of its shapes, with the wide band and with many bands."""
     monkeypatch.setenv("PHDE_SSSP_CTAS", ctas)
     if delta:
         monkeypatch.setenv("PHDE_SSSP_DELTA", delta)
