@@ -725,9 +725,10 @@ __global__ void __launch_bounds__(KB_THREADS) kcenters_block_kernel(KbArgs a) {
 // see the same total: 0 ends the pass, more than `limit` (a wide level: the whole grid is faster) leaves the
 // kernel, and kcenters_bfs_kernel, launched after it, goes on from the pass that was not finished.
 // Sources, history and duplicate fix-up as in kcenters_bfs_kernel; distances are unique, so the results are equal.
-// Measured (16 CTAs of 512 threads): a level is 3100 clocks on the 125 x 125 mesh (expand 840, barrier with the
-// ORs in flight 1240, scan 990), 4000 on a 150k-vertex 2-D geometric graph; whole layouts 21.4 -> 6.7 ms and
-// 139 -> 43 ms.  8 CTAs: 7.7 and 54 ms; 256 threads: 7.2 and 50 ms.
+// Measured (16 CTAs of 512 threads): a level was 3100 clocks on the 125 x 125 mesh (expand 840, barrier with the ORs in
+// flight 1240, scan 990) and 4000 on a 150k-vertex 2-D geometric graph before the words were dealt to the scanning
+// warps in turn and the listed rows prefetched (4 % less); whole layouts 21.4 -> 6.4 ms and 139 -> 40.6 ms.
+// 8 CTAs: 7.7 and 54 ms; 256 threads: 7.2 and 50 ms; 1024 threads: 5 and 2 % slower.
 struct KlArgs {
   const int64_t *off;
   const uint32_t *adj;
@@ -785,15 +786,22 @@ struct KlLevel {
   const uint32_t *rs;    // row starts, 33 per word (null: from off)
   const uint2 *list;     // the CTA's frontier: row start and length
   uint32_t next;         // shared address of the level's next-frontier words
-  uint32_t cnt, rank, cmask, clog;
+  uint32_t cnt, rank, cmask, clog, pitch;
 };
+
+// Place of the CTA's word w in its bitmaps: the words of scanning warp w % KL_WARPS side by side, so that neighbouring
+// words, which a wave fills together, go to different warps.
+constexpr int KL_WARPS = KL_THREADS / 32;
+__device__ __forceinline__ uint32_t kl_place(uint32_t w, uint32_t pitch) {
+  return (w % KL_WARPS) * pitch + w / KL_WARPS;
+}
 
 __device__ __forceinline__ uint32_t kl_vertex(const KlLevel &l, uint32_t x) {
   return (((x >> 5) << l.clog | l.rank) << 5) | (x & 31);
 }
 __device__ __forceinline__ void kl_send(const KlLevel &l, uint32_t v) {
   const uint32_t w = v >> 5;
-  remote_or(map_rank(l.next + ((w >> l.clog) << 2), w & l.cmask), 1u << (v & 31));
+  remote_or(map_rank(l.next + (kl_place(w >> l.clog, l.pitch) << 2), w & l.cmask), 1u << (v & 31));
 }
 __device__ __forceinline__ uint2 kl_row(const KlLevel &l, uint32_t x) {
   if (l.rs) {
@@ -837,7 +845,7 @@ __device__ __forceinline__ ull cluster_max(ull mine, ull *slots, uint32_t rank, 
   return m;
 }
 
-__global__ void __launch_bounds__(KL_THREADS) kcenters_cluster_kernel(KlArgs a) {
+__global__ void __launch_bounds__(KL_THREADS, 1) kcenters_cluster_kernel(KlArgs a) {
   extern __shared__ uint32_t kl_smem[];  // list, visited, next[2], (row starts), history
   __shared__ uint32_t s_counts[2][KL_MAX_CLUSTER];
   __shared__ ull s_keys[KL_MAX_CLUSTER], s_sums[KL_MAX_CLUSTER], s_fix[KL_MAX_CLUSTER];
@@ -846,7 +854,7 @@ __global__ void __launch_bounds__(KL_THREADS) kcenters_cluster_kernel(KlArgs a) 
   __shared__ ull red[32];
   const uint32_t tid = threadIdx.x, rank = cluster_rank(), C = cluster_size();
   const int words = a.words, warp = tid >> 5, lane = tid & 31;
-  const int chunk = min(32, (words + KL_THREADS / 32 - 1) / (KL_THREADS / 32));  // words of a warp in one step of a scan
+  const int pitch = words / KL_WARPS;  // words of a warp (words is a multiple of KL_WARPS)
   uint32_t *vis = kl_smem + 2 * KL_LIST, *next = vis + words;
   uint32_t *rs = vis + 3 * words;
   uint2 *list = (uint2 *)kl_smem;
@@ -859,6 +867,7 @@ __global__ void __launch_bounds__(KL_THREADS) kcenters_cluster_kernel(KlArgs a) 
   l.rank = rank;
   l.cmask = C - 1;
   l.clog = 31 - __clz((int)C);
+  l.pitch = (uint32_t)pitch;
   if (a.rows)
     for (int i = tid; i < 33 * words; i += KL_THREADS) {
       const int64_t v = ((((int64_t)(i / 33) << l.clog) | rank) << 5) + i % 33;
@@ -876,7 +885,7 @@ __global__ void __launch_bounds__(KL_THREADS) kcenters_cluster_kernel(KlArgs a) 
     if (tid == 0) s_long[1] = mine;
     __syncthreads();
     if (tid == 0 && mine) {
-      vis[sx >> 5] = 1u << (sx & 31);
+      vis[kl_place(sx >> 5, l.pitch)] = 1u << (sx & 31);
       list[0] = kl_row(l, sx);
       Dp[src] = 0;
     }
@@ -925,16 +934,16 @@ __global__ void __launch_bounds__(KL_THREADS) kcenters_cluster_kernel(KlArgs a) 
       // the new vertices of each word are listed by a warp together (a lane per bit): a wave that runs along the
       // numbering fills whole words, and one thread per word took 2000-2700 clocks a level
       uint32_t *nx = next + par * words;
-      for (int w0 = warp * chunk; w0 < words; w0 += (KL_THREADS / 32) * chunk) {
-        const int w = w0 + lane;
+      for (int i0 = 0; i0 < pitch; i0 += 32) {
+        const int at0 = warp * pitch + i0 + lane;
         uint32_t nw = 0, slot = 0;
-        if (lane < chunk && w < words) {
-          nw = nx[w];
+        if (i0 + lane < pitch) {
+          nw = nx[at0];
           if (nw) {
-            nx[w] = 0u;
-            const uint32_t seen = vis[w];
+            nx[at0] = 0u;
+            const uint32_t seen = vis[at0];
             nw &= ~seen;
-            vis[w] = seen | nw;
+            vis[at0] = seen | nw;
             if (nw) slot = atomicAdd(&s_cnt[par], (uint32_t)__popc(nw));
           }
         }
@@ -944,12 +953,13 @@ __global__ void __launch_bounds__(KL_THREADS) kcenters_cluster_kernel(KlArgs a) 
           const uint32_t bits = __shfl_sync(PHDE_FULL_MASK, nw, j);
           const uint32_t at = __shfl_sync(PHDE_FULL_MASK, slot, j) + __popc(bits & ((1u << lane) - 1u));
           if (!((bits >> lane) & 1u)) continue;
-          const uint32_t y = ((uint32_t)(w0 + j) << 5) | lane;
+          const uint32_t y = (((uint32_t)(i0 + j) * KL_WARPS + warp) << 5) | lane;
           Dp[kl_vertex(l, y)] = (int32_t)L;
           if (at >= KL_LIST) continue;
           const uint2 row = kl_row(l, y);
           list[at] = row;
           longrow |= row.y > KL_ROW;
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(a.adj + row.x));  // read after the block's barrier
         }
         if (longrow) s_long[par] = 1u;
       }
@@ -979,7 +989,7 @@ __global__ void __launch_bounds__(KL_THREADS) kcenters_cluster_kernel(KlArgs a) 
         const int i = i0 + t * KL_THREADS;
         const int64_t v = ((((int64_t)(i >> 5) << l.clog) | rank) << 5) | (i & 31);
         const bool ok = i < 32 * words && v < a.n;
-        const bool seen = ok && ((vis[i >> 5] >> (i & 31)) & 1u);
+        const bool seen = ok && ((vis[kl_place(i >> 5, l.pitch)] >> (i & 31)) & 1u);
         if (ok && !seen) {
           bad = 1;
           Dp[v] = -1;
@@ -1085,7 +1095,7 @@ static int run_cluster_passes(phde_ctx *ctx, const KcArgs &g, const int64_t **re
   PHDE_CK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   for (;; C /= 2) {  // 16 CTAs, or 8 where the device cannot place 16
     if (C < 8) return PHDE_OK;
-    a.words = (int)((g.W + C - 1) / C);
+    a.words = (int)((g.W + C * KL_WARPS - 1) / (C * KL_WARPS)) * KL_WARPS;
     const size_t fixed = sizeof(uint2) * KL_LIST + sizeof(uint32_t) * (size_t)((g.P + 3) & ~3);
     const size_t room = 224 * 1024;
     a.rows = fixed + sizeof(uint32_t) * 36 * (size_t)a.words <= room;
