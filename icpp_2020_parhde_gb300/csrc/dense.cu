@@ -864,48 +864,73 @@ __global__ void centre_kernel(const int32_t *D, int64_t n, int k, const ull *col
   }
 }
 
-// X[i + t*n] = sum_q M[i,q] * Y[q + t*k]; per-block partial sums of squares per coordinate.
-// X[:, t] = S Y[:, t], FP64: a block stages blockDim.x consecutive rows of S (one contiguous range, read
-// coalesced) into shared memory at a padded stride, then a thread per row forms up to CO_MAXC coordinates,
-// each summed over the row's k entries in order with fused multiply-adds (more coordinates run in groups).
+// X[i + t*n] = sum_q M[i,q] * Y[q + t*k]; per-block partial sums of squares per coordinate.  FP64: a thread per row of
+// S, read straight from global memory (a row is contiguous, its sectors come back from L1), forms up to CO_MAXC
+// coordinates, each summed over the row's k entries in order with fused multiply-adds.  Bound by the FP64 pipe, which
+// a predicated-off FMA holds like any other: with the coordinates' count known at run time only, all eight were issued
+// for two -- 256^3 grid, k = 20, c = 2: 5.54 -> 1.23 ms (1.16 is the pipe's time); R-MAT 20, k = 50, c = 3: 0.68 -> 0.19.
 constexpr int CO_MAXC = 8;
+template <int NC>
+__device__ __forceinline__ void coords_row(const double *row, const double *Ys, int k, double (&sv)[CO_MAXC]) {
+  double s[NC];
+#pragma unroll
+  for (int t = 0; t < NC; t++) s[t] = 0;
+  if ((k & 1) == 0) {  // rows of whole 16-byte pairs
+#pragma unroll 4
+    for (int q = 0; q < k; q += 2) {
+      const double2 m = __ldg((const double2 *)(row + q));
+#pragma unroll
+      for (int t = 0; t < NC; t++) s[t] = fma(m.y, Ys[q + 1 + t * k], fma(m.x, Ys[q + t * k], s[t]));
+    }
+  } else {
+#pragma unroll 4
+    for (int q = 0; q < k; q++) {
+      const double m = __ldg(row + q);
+#pragma unroll
+      for (int t = 0; t < NC; t++) s[t] = fma(m, Ys[q + t * k], s[t]);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < NC; t++) sv[t] = s[t];
+}
+
+// A thread per row, read straight from global memory.  The columns of Y go by groups of up to CO_MAXC, a group's
+// count at compile time up to 3 (2 and 3 coordinates are what layouts ask for).
 __global__ void __launch_bounds__(128) coords_kernel(const double *M, const double *Y, int64_t n, int k, int c,
                                                      double *X, double *part) {
-  extern __shared__ double csm[];  // the group's Ys[q + t * k], then the row tile [blockDim.x][k + 1]
+  extern __shared__ double csm[];  // the group's Ys[q + t * k]
   __shared__ double red[32];
-  const int rows = blockDim.x, kp = k + 1;
-  double *Ys = csm, *tile = csm + (size_t)k * CO_MAXC;
+  const int rows = blockDim.x;
+  double *Ys = csm;
   for (int t0 = 0; t0 < c; t0 += CO_MAXC) {
     const int cg = min(CO_MAXC, c - t0);
-    __syncthreads();  // the previous group's last tile read
-    for (int i = threadIdx.x; i < k * cg; i += blockDim.x) Ys[i] = Y[(int64_t)t0 * k + i];
+    __syncthreads();  // the previous group's Ys read
+    for (int i = threadIdx.x; i < k * CO_MAXC; i += blockDim.x) Ys[i] = i < k * cg ? Y[(int64_t)t0 * k + i] : 0.0;
+    __syncthreads();
     double ss[CO_MAXC];
 #pragma unroll
     for (int t = 0; t < CO_MAXC; t++) ss[t] = 0;
     for (int64_t i0 = (int64_t)blockIdx.x * rows; i0 < n; i0 += (int64_t)gridDim.x * rows) {
-      const int nr = (int)min((int64_t)rows, n - i0);
-      __syncthreads();  // Ys written (first tile), or the previous tile read
-      const double *src = M + i0 * k;
-      for (int e = threadIdx.x; e < nr * k; e += blockDim.x) tile[(e / k) * kp + e % k] = src[e];
-      __syncthreads();
-      if ((int)threadIdx.x < nr) {
-        const double *row = tile + threadIdx.x * kp;
-        double sv[CO_MAXC];
+      const int64_t i = i0 + threadIdx.x;
+      if (i >= n) continue;
+      double sv[CO_MAXC];
 #pragma unroll
-        for (int t = 0; t < CO_MAXC; t++) sv[t] = 0;
-        for (int q = 0; q < k; q++) {
-          const double m = row[q];
+      for (int t = 0; t < CO_MAXC; t++) sv[t] = 0;
+      const double *row = M + i * k;
+      if (cg == 1)
+        coords_row<1>(row, Ys, k, sv);
+      else if (cg == 2)
+        coords_row<2>(row, Ys, k, sv);
+      else if (cg == 3)
+        coords_row<3>(row, Ys, k, sv);
+      else
+        coords_row<CO_MAXC>(row, Ys, k, sv);
 #pragma unroll
-          for (int t = 0; t < CO_MAXC; t++)
-            if (t < cg) sv[t] = fma(m, Ys[q + t * k], sv[t]);
+      for (int t = 0; t < CO_MAXC; t++)
+        if (t < cg) {
+          X[i + (int64_t)(t0 + t) * n] = sv[t];
+          ss[t] = fma(sv[t], sv[t], ss[t]);
         }
-#pragma unroll
-        for (int t = 0; t < CO_MAXC; t++)
-          if (t < cg) {
-            X[i0 + threadIdx.x + (int64_t)(t0 + t) * n] = sv[t];
-            ss[t] = fma(sv[t], sv[t], ss[t]);
-          }
-      }
     }
     for (int t = 0; t < cg; t++) {  // cg is uniform: every thread takes part in each block sum
       const double tot = block_sum(ss[t], red);
@@ -914,8 +939,6 @@ __global__ void __launch_bounds__(128) coords_kernel(const double *M, const doub
   }
 }
 
-// X[:, t] /= ||X[:, t]||: each block sums the per-block partials itself (block-wide, fixed order), then scales;
-// block 0 also reports ||X[:, t]||^2 before the scaling (norm2, optional).
 __global__ void scale_coords_kernel(double *X, int64_t n, int c, const double *part, int nparts, double *norm2) {
   __shared__ double inv[PHDE_MAX_K];
   __shared__ double red[32];
@@ -1205,14 +1228,12 @@ int phde_coords(phde_ctx *ctx, const double *M, const double *Y, int k, int c, d
     PHDE_LAUNCHED(ctx);
     return PHDE_OK;
   }
-  // row tiles of 128 rows (64 for k > 100): at most (256 * 8 + 64 * 257) * 8 bytes of shared memory
+  // blocks of 128 rows, 64 for k > 100
   const int rows = k <= 100 ? 128 : 64;
   const int grid = grid_for(ctx, ctx->n, rows, 8);
   double *part = (double *)phde_buf(ctx, "coords.part", sizeof(double) * grid * (size_t)c);
   if (!part) return PHDE_ERR_OOM;
-  const size_t smem = sizeof(double) * ((size_t)k * CO_MAXC + (size_t)rows * (k + 1));
-  PHDE_CK(ctx, cudaFuncSetAttribute(coords_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)std::max<size_t>(smem, 48 * 1024)));
+  const size_t smem = sizeof(double) * (size_t)k * CO_MAXC;
   coords_kernel<<<grid, rows, smem, ctx->stream>>>(M, Y, ctx->n, k, c, X, part);
   PHDE_LAUNCHED(ctx);
   scale_coords_kernel<<<grid_for(ctx, ctx->n * c, 256), 256, 0, ctx->stream>>>(X, ctx->n, c, part, grid, norm2);
