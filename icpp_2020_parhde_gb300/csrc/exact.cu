@@ -36,7 +36,8 @@
 namespace {
 
 constexpr int ZG_THREADS = 256;
-constexpr int ZG_ROWS = 32;   // rows per staged slab
+constexpr int ZG_ROWS = 32;   // rows per staged slab (one warp's lanes)
+constexpr unsigned ZG_LIGHT = 1u << 20;  // degrees above it take the row-by-row bounds
 constexpr int LG_THREADS = 256;
 constexpr int LG_ITEMS = 64;  // rows / chunks per slab
 constexpr int64_t LG_LIGHT = 16;  // rows of at most this many neighbours are gathered by one lane group
@@ -56,6 +57,22 @@ __device__ __forceinline__ void tile_of(int t, int qb0, int qb1, int &pb, int &q
     }
     t -= b + 1;
   }
+}
+
+// Predicated loads (0 where off): unlike a load under a branch, several of them are in flight at once.
+__device__ __forceinline__ int ld_if(const int32_t *p, bool on) {
+  int v;
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.s32 %0, 0;\n\t@p ld.global.nc.s32 %0, [%1];\n\t}"
+      : "=r"(v)
+      : "l"(p), "r"((unsigned)on));
+  return v;
+}
+__device__ __forceinline__ int ld_if(const uint16_t *p, bool on) {
+  unsigned short v;
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u16 %0, 0;\n\t@p ld.global.nc.u16 %0, [%1];\n\t}"
+      : "=h"(v)
+      : "l"(p), "r"((unsigned)on));
+  return (int)v;
 }
 
 __device__ __forceinline__ double gsym(const ull *G, int ld, int p, int q) {
@@ -81,19 +98,26 @@ struct ZgArgs {
 // column into one word (dp4a: four rows of Z^T Z per instruction) and ys2[h][col] packs deg * z of rows 2h, 2h+1
 // as two 16-bit halves (dp2a against the bytes of zs4: two rows of Z^T D Z per instruction).  Rows whose
 // deg * z does not fit 16 bits take the one-row 32-bit path.  Every sum is still exact.
-__global__ void __launch_bounds__(ZG_THREADS) zgram_kernel(ZgArgs a) {
+//
+// Distances above a byte are bound by the 32-bit multiply-adds (36 a row and tile).  A slab whose products all
+// fit 32 bits together (sum of degrees * largest distance^2) runs its rows without a bound per row; the slab is
+// loaded with eight predicated loads a thread in flight; the block is no wider than the tiles there are and
+// takes 80 registers, so four are resident.  8.0 M vertices, 76 columns: 11.1 -> 7.8 ms.
+__global__ void __launch_bounds__(ZG_THREADS, 3) zgram_kernel(ZgArgs a) {
   if (a.wide_only && __ldg(a.wide_only) <= 255u) return;  // uniform: the quad-layout kernel formed them
   extern __shared__ int zsm[];  // [ZG_ROWS][S], zs4[ZG_ROWS/4][S], ys2[ZG_ROWS/2][S], then the record columns
-  __shared__ unsigned s_deg[ZG_ROWS];
-  __shared__ ull red[32];
+  __shared__ unsigned s_deg[ZG_ROWS], s_mz[ZG_THREADS / 32], s_md, s_sd;
   const int S = a.c1 + 4;
   uint32_t *zs4 = (uint32_t *)zsm + ZG_ROWS * S, *ys2 = zs4 + (ZG_ROWS / 4) * S;
   int *s_rmap = (int *)(ys2 + (ZG_ROWS / 2) * S);
+  constexpr int U = 8;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x & 31, nw = blockDim.x / 32;
+  unsigned top_z = 0, top_d = 0;
   const int P0 = a.src.P0;
   // Z columns [0, nd) are the ones column and D columns; [nd, c1) record columns (or padding beyond P)
-  const int nd = min(a.c1, P0 + 1), nr = a.c1 - nd;
-  for (int j = threadIdx.x; j < nr; j += ZG_THREADS) s_rmap[j] = nd + j <= a.P ? a.src.rmap[nd + j - 1 - P0] : -1;
-  const int t = blockIdx.y * ZG_THREADS + threadIdx.x;
+  const int nd = min(a.c1, P0 + 1), nr = a.c1 - nd, nseg = (nr + 31) / 32 * ZG_ROWS;
+  for (int j = threadIdx.x; j < nr; j += blockDim.x) s_rmap[j] = nd + j <= a.P ? a.src.rmap[nd + j - 1 - P0] : -1;
+  const int t = blockIdx.y * blockDim.x + threadIdx.x;
   int pb, qb;
   tile_of(t, a.c0 / 4, a.c1 / 4, pb, qb);
   const bool active = t < a.ntiles && pb >= 0;
@@ -122,38 +146,64 @@ __global__ void __launch_bounds__(ZG_THREADS) zgram_kernel(ZgArgs a) {
   for (int64_t i0 = r0; i0 < r1; i0 += ZG_ROWS) {
     const int rows = (int)min((int64_t)ZG_ROWS, r1 - i0);
     __syncthreads();  // previous slab consumed
-    unsigned mz = 0, md = 0;
-    for (int e = threadIdx.x; e < ZG_ROWS * nd; e += ZG_THREADS) {  // consecutive threads: rows of a column
-      const int col = e / ZG_ROWS, r = e - col * ZG_ROWS;
-      int v = 0;
-      if (r < rows) v = col == 0 ? 1 : (col - 1 < a.P ? a.src.D[(int64_t)(col - 1) * a.n + i0 + r] : 0);
-      zsm[r * S + col] = v;
-      mz = max(mz, (unsigned)v);
+    unsigned mz = 0;  // an unreached vertex (-1) reads as the largest value: refused by the host
+    // D columns: a warp per column, its lanes the slab's rows
+    for (int cb = warp; cb < nd; cb += nw * U) {
+      int v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int col = cb + u * nw;
+        v[u] = ld_if(a.src.D + (int64_t)(col - 1) * a.n + i0 + lane, col > 0 && col < nd && col - 1 < a.P && lane < rows);
+        if (col == 0 && lane < rows) v[u] = 1;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (cb + u * nw < nd) {
+          zsm[lane * S + cb + u * nw] = v[u];
+          mz = max(mz, (unsigned)v[u]);
+        }
     }
-    for (int e = threadIdx.x; e < ZG_ROWS * nr; e += ZG_THREADS) {  // consecutive threads: columns of a row
-      const int r = e / nr, j = e - r * nr;
-      const int rc = s_rmap[j];
-      const int v = r < rows && rc >= 0 ? (int)a.src.R[(i0 + r) * a.src.RW + rc] - 1 : 0;
-      zsm[r * S + nd + j] = v;
-      mz = max(mz, (unsigned)v);
+    // record columns: a warp per (row, 32 columns)
+    for (int f = warp; f < nseg; f += nw * U) {
+      int v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int g = f + u * nw, r = g & (ZG_ROWS - 1), j = (g / ZG_ROWS) * 32 + lane;
+        const int rc = g < nseg && j < nr && r < rows ? s_rmap[j] : -1;
+        v[u] = ld_if(a.src.R + i0 * a.src.RW + (r * a.src.RW + rc), rc >= 0) - (rc >= 0);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int g = f + u * nw, r = g & (ZG_ROWS - 1), j = (g / ZG_ROWS) * 32 + lane;
+        if (g < nseg && j < nr) {
+          zsm[r * S + nd + j] = v[u];
+          mz = max(mz, (unsigned)v[u]);
+        }
+      }
     }
-    if (threadIdx.x < ZG_ROWS) {
-      const int r = threadIdx.x;
-      const unsigned d = r < rows ? (unsigned)(a.off[i0 + r + 1] - a.off[i0 + r]) : 0u;
-      s_deg[r] = d;
-      md = d;
+    if (warp == 0) {  // ZG_ROWS == 32: lane r has the slab's row r
+      const unsigned d = lane < rows ? (unsigned)(a.off[i0 + lane + 1] - a.off[i0 + lane]) : 0u;
+      s_deg[lane] = d;
+      const unsigned md = __reduce_max_sync(0xffffffffu, d);
+      const unsigned sd = __reduce_add_sync(0xffffffffu, lane < rows ? max(min(d, ZG_LIGHT), 1u) : 0u);
+      if (lane == 0) {
+        s_md = md;
+        s_sd = sd;
+      }
     }
-    const ull mzs = block_max_u64((ull)mz, red);
-    const ull mds = block_max_u64((ull)md, red);
-    if (threadIdx.x == 0) {
-      atomicMax(a.maxz, (unsigned)mzs);
-      atomicMax(a.maxz + 1, (unsigned)mds);
-    }
+    mz = __reduce_max_sync(0xffffffffu, mz);
+    if (lane == 0) s_mz[warp] = mz;
+    __syncthreads();
+    unsigned mzw = 0;
+    for (int w = 0; w < nw; w++) mzw = max(mzw, s_mz[w]);
+    const ull mzs = mzw;
+    top_z = max(top_z, mzw);
+    top_d = max(top_d, s_md);
     const ull mz2 = mzs * mzs;
     const bool bytes = mzs <= 255;  // uniform: the slab's distances fit a byte
     if (bytes) {
       // pack (rows past the end and rows for the 32-bit path pack as zeros)
-      for (int e = threadIdx.x; e < (ZG_ROWS / 4) * a.c1; e += ZG_THREADS) {
+      for (int e = threadIdx.x; e < (ZG_ROWS / 4) * a.c1; e += blockDim.x) {
         const int q = e / a.c1, col = e - q * a.c1;
         uint32_t w = 0;
 #pragma unroll
@@ -163,7 +213,7 @@ __global__ void __launch_bounds__(ZG_THREADS) zgram_kernel(ZgArgs a) {
         }
         zs4[q * S + col] = w;
       }
-      for (int e = threadIdx.x; e < (ZG_ROWS / 2) * a.c1; e += ZG_THREADS) {
+      for (int e = threadIdx.x; e < (ZG_ROWS / 2) * a.c1; e += blockDim.x) {
         const int h = e / a.c1, col = e - h * a.c1;
         uint32_t w = 0;
 #pragma unroll
@@ -206,6 +256,34 @@ __global__ void __launch_bounds__(ZG_THREADS) zgram_kernel(ZgArgs a) {
             }
         }
       }
+    }
+    if (!bytes && mzs <= 65535 && s_md <= ZG_LIGHT && (ull)s_sd * mz2 < B32) {
+      // the whole slab's products fit 32 bits: no bound per row (rows past the end are zeros)
+      if (run + (ull)s_sd * mz2 >= B32) {
+        flush();
+        run = 0;
+      }
+      run += (ull)s_sd * mz2;
+      if (active) {
+        const int *zr = zsm;
+#pragma unroll 2
+        for (int r = 0; r < ZG_ROWS; r++, zr += S) {
+          const unsigned d = s_deg[r];
+          const uint4 zp = *(const uint4 *)(zr + 4 * pb);
+          const uint4 zq = *(const uint4 *)(zr + 4 * qb);
+          const uint32_t p4[4] = {zp.x, zp.y, zp.z, zp.w}, q4[4] = {zq.x, zq.y, zq.z, zq.w};
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const uint32_t y = p4[i] * d;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              aI[i][j] += p4[i] * q4[j];
+              aD[i][j] += y * q4[j];
+            }
+          }
+        }
+      }
+      continue;
     }
     for (int r = 0; r < rows; r++) {
       const unsigned d = s_deg[r];
@@ -251,6 +329,10 @@ __global__ void __launch_bounds__(ZG_THREADS) zgram_kernel(ZgArgs a) {
         }
       }
     }
+  }
+  if (threadIdx.x == 0) {
+    atomicMax(a.maxz, top_z);
+    atomicMax(a.maxz + 1, top_d);
   }
   flush();
 }
@@ -835,7 +917,11 @@ __global__ void __launch_bounds__(CF_THREADS, 1) coef_kernel(CoefArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// Z_acc[i][t] = D[acc_idx[t] - 1][i] for t < k, 0 for k <= t < kp; 16 bytes per store.
+// Z_acc[i][t] = D[acc_idx[t] - 1][i] for t < k, 0 for k <= t < kp; 16 bytes per store.  kp / (16 / sizeof(T)) is
+// a power of two.
+// Bound by the loads' L1 wavefronts.  Records are row-major, so their lanes take a row's stores in turn: a load
+// touches the lines of 4 rows (16-bit, k <= 64) where lanes on 32 rows touch 32.  Columns of D are column-major
+// and keep their lanes along the rows.  8.0 M vertices, k = 64, 16-bit: 6.2 -> 0.87 ms (1.0 GB written, 1.0 GB read).
 template <typename T>
 __global__ void pack_kernel(ZSrc src, int64_t n, const int *acc_idx, int k, int kp, T *Z) {
   __shared__ int s_col[PHDE_MAX_K];
@@ -847,19 +933,30 @@ __global__ void pack_kernel(ZSrc src, int64_t n, const int *acc_idx, int k, int 
   }
   __syncthreads();
   constexpr int V = 16 / sizeof(T);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    for (int t0 = 0; t0 < kp; t0 += V) {
-      union {
-        uint4 u;
-        T v[V];
-      } w;
+  auto store = [&](int64_t i, int t0) {
+    union {
+      uint4 u;
+      T v[V];
+    } w;
+    int d[V], r[V];
 #pragma unroll
-      for (int j = 0; j < V; j++) {
-        const int col = s_col[t0 + j];
-        w.v[j] = col < 0 ? (T)0 : s_rec[t0 + j] ? (T)(src.R[i * src.RW + col] - 1) : (T)src.D[(int64_t)col * n + i];
-      }
-      *(uint4 *)(Z + i * kp + t0) = w.u;
+    for (int j = 0; j < V; j++) {
+      const int col = s_col[t0 + j];
+      const bool on = col >= 0, rec = s_rec[t0 + j];
+      r[j] = ld_if(src.R + i * src.RW + col, on && rec) - (on && rec);
+      d[j] = ld_if(src.D + (int64_t)col * n + i, on && !rec);
     }
+#pragma unroll
+    for (int j = 0; j < V; j++) w.v[j] = (T)(r[j] + d[j]);
+    *(uint4 *)(Z + i * kp + t0) = w.u;
+  };
+  const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  if (src.R) {
+    const int lg = 31 - __clz(kp / V);
+    for (int64_t e = first; e < n << lg; e += step) store(e >> lg, (int)(e & ((1 << lg) - 1)) * V);
+  } else {
+    for (int64_t i = first; i < n; i += step)
+      for (int t0 = 0; t0 < kp; t0 += V) store(i, t0);
   }
 }
 
@@ -1550,11 +1647,12 @@ static int exact_zgram(phde_ctx *ctx, const ZSrc &src, int P, int c0, int c1, ul
     if (byte_state == 1) return PHDE_OK;
   }
   if (src.lvl) return PHDE_OK;  // level mode: distances above 254 cannot occur; an unreached one (maxz) is refused
-  const int gy = (ntiles + ZG_THREADS - 1) / ZG_THREADS;
+  const int zt = std::min(ZG_THREADS, std::max(128, (ntiles + 31) / 32 * 32));
+  const int gy = (ntiles + zt - 1) / zt;
   const size_t smem = sizeof(int) * ((ZG_ROWS + ZG_ROWS / 4 + ZG_ROWS / 2) * (size_t)(c1 + 4) + c1);
   PHDE_CK(ctx, cudaFuncSetAttribute(zgram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
-  PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, zgram_kernel, ZG_THREADS, smem));
+  PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, zgram_kernel, zt, smem));
   per_sm = std::max(1, std::min(per_sm, 4));
   const int gx = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)ctx->nsm * per_sm / gy,
                                                               (ctx->n + ZG_ROWS - 1) / ZG_ROWS));
@@ -1571,7 +1669,7 @@ static int exact_zgram(phde_ctx *ctx, const ZSrc &src, int P, int c0, int c1, ul
   a.ld = ld;
   a.maxz = maxz;
   a.wide_only = byte_state < 0 ? maxz : nullptr;
-  zgram_kernel<<<dim3(gx, gy), ZG_THREADS, smem, ctx->stream>>>(a);
+  zgram_kernel<<<dim3(gx, gy), zt, smem, ctx->stream>>>(a);
   PHDE_LAUNCHED(ctx);
   return PHDE_OK;
 }

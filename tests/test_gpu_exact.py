@@ -144,3 +144,45 @@ def test_exact_rejected_for_other_algorithms(gpu_ctx):
     with pytest.raises(ParHDEError) as e:
         gpu_ctx.layout("PivotMDS", "Kcenters", 5, 2, precision="exact")
     assert e.value.status == -1
+
+
+def tailed(core, tails, shortest, hub_leaves=0, seed=1):
+    """A ring of `core` vertices with random chords, a tail (path) of shortest + j vertices on `tails` of them, and
+    hub_leaves vertices of degree one on vertex 0: distances above 255 with well-separated columns."""
+    rng = np.random.default_rng(seed)
+    ring = np.arange(core, dtype=np.int64)
+    u, v = [ring, ring], [(ring + 1) % core, rng.permutation(core).astype(np.int64)]
+    n = core
+    for j in range(tails):
+        L = shortest + j
+        ids = np.arange(n, n + L, dtype=np.int64)
+        u.append(np.concatenate([[rng.integers(core)], ids[:-1]]))
+        v.append(ids)
+        n += L
+    u.append(np.zeros(hub_leaves, dtype=np.int64))
+    v.append(np.arange(n, n + hub_leaves, dtype=np.int64))
+    n += hub_leaves
+    u, v = np.concatenate(u), np.concatenate(v)
+    keep = u != v
+    return graphs._csr_from_undirected(n, *graphs._unique_undirected(n, u[keep], v[keep])[:2])
+
+
+# The 16-bit columns: record columns (Learned) and columns of D (Kcenters), k on both sides of a packed row of
+# 64, one and two CTAs of tiles, a ragged last slab, and a row too heavy for the slab's common bound.
+# Tolerances: ten times what the C oracle and the numpy restatement, both FP64, differ by on the same graph and
+# Kcenters sources (basis 2.2e-11, never below 1e-9 here, and Gram 4.5e-9 for the tails; 8.7e-9 and 2.2e-7 for the hub).
+@pytest.mark.parametrize("strategy,make,k,btol,mtol", [
+    ("Learned", lambda: tailed(501, 72, 270), 64, 1e-9, 5e-8),
+    ("Learned", lambda: tailed(501, 72, 270), 20, 1e-9, 5e-8),
+    ("Learned", lambda: tailed(400, 112, 258), 100, 1e-9, 5e-8),
+    ("Kcenters", lambda: tailed(501, 72, 270), 61, 1e-9, 5e-8),
+    ("Kcenters", lambda: tailed(50, 6, 300, hub_leaves=(1 << 20) + 5), 5, 1e-7, 3e-6),
+], ids=["records-k64", "records-k20", "records-k100", "columns-k61", "heavy-hub"])
+def test_exact_wide_distances(gpu_ctx, strategy, make, k, btol, mtol):
+    g = make()
+    gpu_ctx.upload(g)
+    r = gpu_ctx.layout("ParHDE", strategy, k, 2, precision="exact", eig="exact", extra=True)
+    X, S, M, na, nd = orc.hde_from_sources(g, r.sources, k, 2)
+    assert r.stats["naccepted"] == na and r.stats["ndiscarded"] == nd
+    np.testing.assert_allclose(r.basis, S, rtol=0, atol=btol)
+    np.testing.assert_allclose(r.gram, M, rtol=0, atol=mtol * np.abs(M).max())
