@@ -16,7 +16,8 @@
 //   coordinates   X_b = S_b Y_b per segment, FP64 column norms per graph.
 // Nothing between the Kcenters launch and the coordinate copy waits on the host, so after the first call
 // the whole sequence is captured once into a CUDA graph and replayed.  The segment length (rows per CTA) is
-// picked by a small autotuner: each candidate length is timed on the caller's own batch at the first call.
+// picked by a small autotuner: the dense stages are timed at each candidate length on the caller's own batch at
+// the first call (the distances do not depend on it).
 // Options outside that pipeline (FP64 or exact arithmetic, k above 32, the power iteration, the other
 // algorithms) lay the graphs out one after another with the single-graph pipeline (layout_per_graph): each
 // graph's CSR is cut out of the union on the device and laid out as if uploaded alone.
@@ -807,7 +808,7 @@ extern "C" int phde_layout_batched(phde_ctx *ctx, const phde_layout_opts *o, dou
     return PHDE_ERR_OOM;
   PHDE_CK(ctx, cudaMemsetAsync(q.edges, 0, sizeof(ull), ctx->stream));
 
-  // ---- segment length: autotuned once per uploaded batch (each candidate timed on this batch) ----
+  // ---- segment length: autotuned once per uploaded batch (dense stages timed on this batch) ----
   auto set_segments = [&](int64_t seg_rows) -> int {
     std::vector<int32_t> g;
     std::vector<int64_t> r0, r1;

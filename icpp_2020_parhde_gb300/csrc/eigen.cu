@@ -7,7 +7,8 @@
 //   reference's sign rule.  The glibc rand() stream (the published TYPE_3 additive-feedback generator) is made
 //   on the host once per context.  The multiply keeps the reference's summation order; the Gram-Schmidt
 //   runs as a wavefront (vector i takes its projection onto vector j at step i+j, when vector j is final),
-//   so its N(N-1)/2 dependent projections take 2N-3 block-synchronous steps.
+//   so its N(N-1)/2 dependent projections take 2N-3 block-synchronous steps; power_cluster_kernel goes by finished
+//   vector instead, N-1 steps over a cluster.
 // jacobi_kernel: exact solve (the LAPACKE_dsyev role of the MKL build): cyclic Jacobi on the symmetric
 //   part with the round-robin pairing, N/2 disjoint rotations per step; eigenvalues ascending; every
 //   eigenvector signed so that its largest-magnitude entry (lowest index on ties) is positive.

@@ -27,6 +27,11 @@
 // Selection (ParHDE.cpp:127-155): min_d[v] = min(min_d[v], d_p[v]); the next source is the vertex of
 // largest min_d, lowest index first (a 64-bit atomicMax on (min_d << 32) | ~v); if that vertex is in
 // the history, the duplicate fix-up takes the highest-index vertex with the same min_d that is not.
+//
+// Three kernels share that rule and give the same bits.  kcenters_bfs_kernel is the grid-wide one above.
+// kcenters_cluster_kernel runs the passes of a sparse graph whose visited bitmap fits a cluster's shared memory:
+// its levels are a few hundred vertices, so the grid barrier was most of their time.  kcenters_block_kernel gives
+// every graph of a large batch its own CTA.
 #include <cstdio>
 #include <cstdlib>
 #include <vector>

@@ -10,6 +10,8 @@
 //   far pile  : improved vertices at or beyond T; when the near frontier empties, T jumps to the band
 //               holding the smallest far distance and the pile is split into the new near frontier and
 //               what stays far.
+// On graphs whose longest row has at most SG_MAX_ROW neighbours the rounds are not edge-balanced: a lane group per
+// frontier vertex reads its row at once (sssp_group_kernel), which spares the owner search.
 // Both lists are de-duplicated with per-vertex stamps.  Shortest-path distances are unique, so the
 // result is bit-exact against the reference whatever the band width or relaxation order.
 #include <algorithm>
