@@ -1239,7 +1239,8 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   void *args[] = {&a};
   cudaEventRecord(ctx->kev[0], ctx->stream);
   a.resume = nullptr;
-  if (B == 0 && (rc = run_cluster_passes(ctx, a, &a.resume))) return rc;
+  // a traced call keeps every pass in the kernel that writes the timeline
+  if (B == 0 && !a.trace && (rc = run_cluster_passes(ctx, a, &a.resume))) return rc;
   PHDE_CK(ctx, cudaLaunchCooperativeKernel((const void *)kcenters_bfs_kernel, dim3(ctx->nsm * per_sm),
                                            dim3(KC_THREADS), args, smem, ctx->stream));
   PHDE_LAUNCHED(ctx);
