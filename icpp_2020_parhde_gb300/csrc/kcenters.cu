@@ -101,6 +101,9 @@ __device__ __forceinline__ void batch_fold(ull *keys, ull *sumsq, int g, ull key
 // The vertices a block finds in a level wait in a shared-memory list (warp-aggregated appends) and go to the grid's
 // queue a block-width at a time: a push is two block barriers and a round trip to the queue's counter, 2700-3200
 // clocks, and one per iteration also kept the iterations' memory trips from overlapping.
+// A level that is one iteration of the grid pushes straight away, its rows' offsets read beside the claim: the list
+// would only add three barriers and a trip (R-MAT 14 and 17, mixed layouts: 2.05 and 2.59 ms with it, 2.02 and 2.42
+// without).
 struct KcList {
   uint32_t *v;
   unsigned *n;
@@ -240,11 +243,12 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
 
       if (!in_bu) {
         const int64_t E = f_edges;
+        const bool once = E <= gstride;
         int since = 0;
         for (int64_t base = gbase; base < E; base += gstride) {
           const int64_t e = base + tid, e0w = base + (tid & ~31);
           bool claimed = false;
-          uint32_t v = 0;
+          uint32_t v = 0, ov = 0, dv = 0;
           if (e0w < E) {  // warp-uniform
             int64_t j = s_off + e;
             if (L != 0 || a.B != 0) {
@@ -255,12 +259,22 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
             if (e < E) {
               v = __ldg(a.adj + j);
               edges_local++;
-              if (Dp[v] == -1 && atomicCAS(Dp + v, -1, L + 1) == -1) {
-                claimed = true;
-                atomicOr(bm_next + (v >> 5), 1u << (v & 31));
+              if (Dp[v] == -1) {
+                if (once) {  // in flight with the CAS
+                  ov = (uint32_t)__ldg(a.off + v);
+                  dv = (uint32_t)__ldg(a.off + v + 1) - ov;
+                }
+                if (atomicCAS(Dp + v, -1, L + 1) == -1) {
+                  claimed = true;
+                  atomicOr(bm_next + (v >> 5), 1u << (v & 31));
+                }
               }
             }
-            list.add(claimed, v);
+            if (!once) list.add(claimed, v);
+          }
+          if (once) {
+            block_push(claimed, v, dv, qout_v, qout_e, octr, &psc, qout_o, ov);
+            break;
           }
           if (++since == full) {  // as many more as the list holds for sure
             since = 0;
@@ -268,8 +282,9 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
             if (__syncthreads_or(s_listed > KC_THREADS)) list.flush(a.off, qout_v, qout_e, qout_o, octr, &psc);
           }
         }
-        list.flush(a.off, qout_v, qout_e, qout_o, octr, &psc);
+        if (!once) list.flush(a.off, qout_v, qout_e, qout_o, octr, &psc);
       } else {
+        const bool once = n <= gstride;
         if (a.smem_bm) {
           // 16 bytes per copy, all of a thread's in flight (word by word: 11k clocks for R-MAT 20's 80 KB)
           for (int64_t w = 4 * (int64_t)tid; w < a.W; w += 4 * (int64_t)blockDim.x) cp_async16(s_bm + w, bm_cur + w);
@@ -282,6 +297,7 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
         for (int64_t base = gbase; base < n; base += gstride) {
           const int64_t v = base + tid;
           bool found = false;
+          uint32_t ov = 0, dv = 0;
           if (v < n && Dp[v] == -1) {
             const int64_t j0 = a.off[v], j1 = a.off[v + 1];
             // four neighbours per round (their adjacency entries, then their bitmap words, all in flight): a
@@ -302,12 +318,18 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
             }
             if (found) {
               Dp[v] = L + 1;
+              ov = (uint32_t)j0;
+              dv = (uint32_t)(j1 - j0);
             }
           }
           // one bitmap word per warp: the warp covers 32 consecutive, 32-aligned vertices
           const uint32_t bal = __ballot_sync(PHDE_FULL_MASK, found);
           const int64_t v0 = v - (tid & 31);
           if ((tid & 31) == 0 && v0 < n) bm_next[v0 >> 5] = bal;
+          if (once) {
+            block_push(found, (uint32_t)v, dv, qout_v, qout_e, octr, &psc, qout_o, ov);
+            break;
+          }
           list.add(found, (uint32_t)v);
           if (++since == full) {
             since = 0;
@@ -315,7 +337,7 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
             if (__syncthreads_or(s_listed > KC_THREADS)) list.flush(a.off, qout_v, qout_e, qout_o, octr, &psc);
           }
         }
-        list.flush(a.off, qout_v, qout_e, qout_o, octr, &psc);
+        if (!once) list.flush(a.off, qout_v, qout_e, qout_o, octr, &psc);
       }
       ull out;
       if (!grid_sync_read(a.gs, a.err, a.timeout_ns, octr, &out)) return;

@@ -263,3 +263,19 @@ def test_sssp_lane_groups_exact(gpu_ctx, monkeypatch, make, ctas, delta):
     d = gpu_ctx.distances(src)
     for i, s in enumerate(src):
         assert np.array_equal(d[:, i], orc.sssp(g, s))
+
+
+@pytest.mark.parametrize("make", [
+    lambda width: graphs.star_graph(width),
+    lambda width: graphs.star_graph(width + 1),
+    lambda width: graphs.rmat(18, seed=4),  # above 24 neighbours a vertex: every level on the whole grid
+], ids=["grid-wide-star", "one-more", "rmat18"])
+def test_kcenters_levels_of_one_and_more_grid_iterations(gpu_ctx, make):
+    """Levels that fit one iteration of the grid push their vertices at once, wider ones list them first: stars
+    whose one level takes exactly the grid's threads and one more, and an R-MAT with levels of both kinds."""
+    import torch
+    g = make(torch.cuda.get_device_properties(0).multi_processor_count * 1024)
+    gpu_ctx.upload(g)
+    D, s = gpu_ctx.kcenters(4, 0)
+    Do, so = orc.kcenters(g, 4, 0, parallel=True)
+    assert np.array_equal(s, so) and np.array_equal(D, Do)
