@@ -124,6 +124,18 @@ void *phde_buf(phde_ctx *ctx, const char *name, size_t bytes) {
   return p;
 }
 
+int phde_allow_smem(phde_ctx *ctx, const void *kernel) {
+  if (ctx->smem_allowed.count(kernel)) return PHDE_OK;
+  int limit = 0;
+  cudaFuncAttributes fa;
+  PHDE_CK(ctx, cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  PHDE_CK(ctx, cudaFuncGetAttributes(&fa, kernel));
+  PHDE_CK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    limit - (int)fa.sharedSizeBytes));
+  ctx->smem_allowed.insert(kernel);
+  return PHDE_OK;
+}
+
 int phde_reset_sync(phde_ctx *ctx) {
   PHDE_CK(ctx, cudaMemsetAsync(ctx->d_sync, 0, sizeof(GridSync), ctx->stream));
   PHDE_CK(ctx, cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));

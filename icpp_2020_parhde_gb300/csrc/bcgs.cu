@@ -332,9 +332,7 @@ int phde_bcgs2_mixed(phde_ctx *ctx, const int32_t *D, int P, const ull *sumsq, c
   PHDE_CK(ctx, cudaMemsetAsync(st, 0, sizeof(int) * 4, ctx->stream));
   const double n_den0 = (double)ctx->nnz;  // n * <u0, D u0> = sum of degrees
   const int g_rows = (int)std::max<int64_t>(1, std::min<int64_t>((n + RT - 1) / RT, (int64_t)ctx->nsm * 8));
-  const size_t upd_smem_max = sizeof(float) * ((size_t)(k + 1) * BB + (size_t)k * ST_LD);
-  PHDE_CK(ctx, cudaFuncSetAttribute(bcgs_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)std::max<size_t>(upd_smem_max, 48 * 1024)));
+  if (int arc = phde_allow_smem(ctx, (const void *)bcgs_update_kernel)) return arc;
   int j = 0;
   int hst[4] = {0, 0, 0, 0};
   for (int rc0 = 0; rc0 < P && j < k; rc0 += BB) {

@@ -4,6 +4,7 @@
 
 #include <cstdint>
 #include <map>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -80,6 +81,7 @@ struct phde_ctx {
   int *d_err = nullptr;
 
   std::map<std::string, std::pair<void *, size_t>> ws;
+  std::set<const void *> smem_allowed;  // kernels phde_allow_smem has seen
   cudaEvent_t ev[8] = {};
   // events bracketing each distance-kernel launch; kev_pending says a pair was recorded
   cudaEvent_t kev[2] = {};
@@ -100,6 +102,11 @@ void phde_collect_kernel_time(phde_ctx *ctx);
 
 // Set the context error message and return `status`.
 int phde_fail(phde_ctx *ctx, int status, const std::string &msg);
+
+// Let launches of `kernel` ask for all the shared memory a block can have beside the kernel's static part.  The limit is
+// the process's, not the context's: set to one launch's own size, another thread's context with a smaller graph would
+// lower it before that launch, which then fails.  Every context sets the same value, once per kernel.
+int phde_allow_smem(phde_ctx *ctx, const void *kernel);
 
 // Grow-only named device buffer; returns nullptr on allocation failure (ctx->err set).
 void *phde_buf(phde_ctx *ctx, const char *name, size_t bytes);

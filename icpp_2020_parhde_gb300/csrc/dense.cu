@@ -1004,7 +1004,7 @@ int phde_cgs(phde_ctx *ctx, const int32_t *D, int P, const ull *sumsq, const dou
   const int64_t n = ctx->n;
   int per_sm = 0;
   const size_t smem = sizeof(double) * (CGS_THREADS / 32) * ((size_t)(k + 2) + 32 * TILE_LD);
-  PHDE_CK(ctx, cudaFuncSetAttribute(cgs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int arc = phde_allow_smem(ctx, (const void *)cgs_kernel)) return arc;
   PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cgs_kernel, CGS_THREADS, smem));
   if (per_sm < 1) return phde_fail(ctx, PHDE_ERR_CUDA, "cgs kernel cannot be resident");
   per_sm = std::min(per_sm, 4);

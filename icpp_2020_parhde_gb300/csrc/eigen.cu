@@ -1038,7 +1038,7 @@ int phde_eigensolve(phde_ctx *ctx, const double *d_M, int N, int c, int largest,
   if (eig == PHDE_EIG_EXACT) {
     if (N <= JS_MAX_N && !getenv("PHDE_JACOBI_GLOBAL")) {
       const size_t jsmem = sizeof(double) * 3 * (size_t)N * (N | 1);
-      PHDE_CK(ctx, cudaFuncSetAttribute(jacobi_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsmem));
+      if (int arc = phde_allow_smem(ctx, (const void *)jacobi_smem_kernel)) return arc;
       // PHDE_EIG_TRACE=1: print the kernel's phase timeline (FP32 sweeps, orthonormalisation, similarity,
       // FP64 sweeps, sort) after the solve
       unsigned long long *tr = getenv("PHDE_EIG_TRACE") ? (unsigned long long *)phde_buf(ctx, "eig.trace", 64) : nullptr;
@@ -1072,7 +1072,7 @@ int phde_eigensolve(phde_ctx *ctx, const double *d_M, int N, int c, int largest,
       else
         power_kernel<false><<<1, EIG_THREADS, 0, ctx->stream>>>(d_M, start, N, d_K, w1, w2, d_evals, st, st + 1, 20000, dd);
     } else {
-      PHDE_CK(ctx, cudaFuncSetAttribute(power_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
+      if (int arc = phde_allow_smem(ctx, (const void *)power_cluster_kernel)) return arc;
       power_cluster_kernel<<<PW_CL, NO <= 8 ? 256 : 512, csmem, ctx->stream>>>(d_M, start, N, d_K, d_evals, st, st + 1, 20000);
     }
   }
@@ -1096,7 +1096,7 @@ int phde_eigensolve_batched(phde_ctx *ctx, const double *d_M, int N, int c, int 
                             double *d_evals, double *d_Y, int *d_st) {
   if (N > JS_MAX_N) return phde_fail(ctx, PHDE_ERR_INVALID, "batched eigensolve: k above the shared-memory limit");
   const size_t jsmem = sizeof(double) * 3 * (size_t)N * (N | 1);
-  PHDE_CK(ctx, cudaFuncSetAttribute(jacobi_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsmem));
+  if (int arc = phde_allow_smem(ctx, (const void *)jacobi_smem_kernel)) return arc;
   jacobi_smem_kernel<<<count, js_threads(N), jsmem, ctx->stream>>>(d_M, N, d_K, d_evals, d_st, d_st + count, 100,
                                                                     nullptr, c, 0);
   PHDE_LAUNCHED(ctx);

@@ -1623,7 +1623,7 @@ static int exact_zgram(phde_ctx *ctx, const ZSrc &src, int P, int c0, int c1, ul
     const int threads = std::min(ZQ_GRAM_THREADS, (ntiles + 31) / 32 * 32);
     const int gy = (ntiles + threads - 1) / threads;
     const size_t smem = sizeof(uint32_t) * 5 * ZQ_QUADS * (size_t)c1 + sizeof(int64_t) * 2 * (ZQ_ROWS + 2);
-    PHDE_CK(ctx, cudaFuncSetAttribute(zgram_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int arc = phde_allow_smem(ctx, (const void *)zgram_q_kernel)) return arc;
     int per_sm = 0;
     PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, zgram_q_kernel, threads, smem));
     per_sm = std::max(1, std::min(per_sm, 4));
@@ -1650,7 +1650,7 @@ static int exact_zgram(phde_ctx *ctx, const ZSrc &src, int P, int c0, int c1, ul
   const int zt = std::min(ZG_THREADS, std::max(128, (ntiles + 31) / 32 * 32));
   const int gy = (ntiles + zt - 1) / zt;
   const size_t smem = sizeof(int) * ((ZG_ROWS + ZG_ROWS / 4 + ZG_ROWS / 2) * (size_t)(c1 + 4) + c1);
-  PHDE_CK(ctx, cudaFuncSetAttribute(zgram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int arc = phde_allow_smem(ctx, (const void *)zgram_kernel)) return arc;
   int per_sm = 0;
   PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, zgram_kernel, zt, smem));
   per_sm = std::max(1, std::min(per_sm, 4));
@@ -1705,7 +1705,7 @@ int phde_exact_orth(phde_ctx *ctx, const ZSrc &src, int P, int k, ExactBasis *eb
   PHDE_CK(ctx, cudaMemcpyAsync(state, st0, sizeof(st0), cudaMemcpyHostToDevice, ctx->stream));
   const size_t csmem0 = sizeof(double) * (2 * (size_t)ld + 2 * (size_t)k + CF_THREADS);
   constexpr size_t CF_SMEM_MAX = 200 * 1024;
-  PHDE_CK(ctx, cudaFuncSetAttribute(coef_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF_SMEM_MAX));
+  if (int arc = phde_allow_smem(ctx, (const void *)coef_kernel)) return arc;
   int c0 = 0, c1 = std::min(ld, (1 + std::min(P, k + std::max(4, k / 8)) + 3) / 4 * 4);
   int hs[4] = {0, 0, 0, 1};
   unsigned hm[2] = {0, 0};
@@ -1813,7 +1813,7 @@ int phde_exact_lap(phde_ctx *ctx, const ZSrc &src, int k, ExactBasis *eb, double
   const size_t smem = sizeof(int) * 2 * LG_ITEMS * (size_t)(kp + 4);
   const int64_t nslab = (n + nch + LG_ITEMS - 1) / LG_ITEMS;
   auto launch = [&](auto kern) -> int {
-    PHDE_CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int arc = phde_allow_smem(ctx, (const void *)kern)) return arc;
     int per_sm = 0;
     PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, LG_THREADS, smem));
     per_sm = std::max(1, per_sm);
@@ -1859,13 +1859,11 @@ int phde_exact_coords(phde_ctx *ctx, const double *M, const double *Y, int k, in
   PHDE_LAUNCHED(ctx);
   const size_t smem = sizeof(uint32_t) * 2 * (size_t)c * kp;
   if (eb->z16) {
-    PHDE_CK(ctx, cudaFuncSetAttribute(coords_fix_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)std::max<size_t>(smem, 48 * 1024)));
+    if (int arc = phde_allow_smem(ctx, (const void *)coords_fix_kernel<uint16_t>)) return arc;
     coords_fix_kernel<uint16_t><<<grid, 128, smem, ctx->stream>>>((const uint16_t *)eb->Z, n, kp, c, whi, wlo, w0,
                                                                   sinv, X, part);
   } else {
-    PHDE_CK(ctx, cudaFuncSetAttribute(coords_fix_kernel<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)std::max<size_t>(smem, 48 * 1024)));
+    if (int arc = phde_allow_smem(ctx, (const void *)coords_fix_kernel<uint8_t>)) return arc;
     coords_fix_kernel<uint8_t><<<grid, 128, smem, ctx->stream>>>((const uint8_t *)eb->Z, n, kp, c, whi, wlo, w0,
                                                                  sinv, X, part);
   }

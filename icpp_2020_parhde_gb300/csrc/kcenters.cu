@@ -1128,7 +1128,7 @@ static int run_cluster_passes(phde_ctx *ctx, const KcArgs &g, const int64_t **re
     a.rows = fixed + sizeof(uint32_t) * 36 * (size_t)a.words <= room;
     smem = fixed + sizeof(uint32_t) * (a.rows ? 36 : 3) * (size_t)a.words;
     if (smem > room) return PHDE_OK;
-    PHDE_CK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (int arc = phde_allow_smem(ctx, (const void *)kernel)) return arc;
     at[0].val.clusterDim.x = C;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(C);
@@ -1204,7 +1204,7 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   const int smem_bm = hist_bytes + bm_bytes <= 98 * 1024;
   const int cap = smem_bm && hist_bytes + bm_bytes > 90 * 1024 ? 2 * KC_THREADS : 4 * KC_THREADS;
   const size_t smem = hist_bytes + sizeof(uint32_t) * cap + (smem_bm ? bm_bytes : 0);
-  PHDE_CK(ctx, cudaFuncSetAttribute(kcenters_bfs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int arc = phde_allow_smem(ctx, (const void *)kcenters_bfs_kernel)) return arc;
   PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kcenters_bfs_kernel, KC_THREADS, smem));
   if (per_sm < 1) return phde_fail(ctx, PHDE_ERR_CUDA, "kcenters kernel cannot be resident");
   per_sm = std::min(per_sm, 2);
@@ -1336,7 +1336,7 @@ int phde_run_bfs_batched_blocks(phde_ctx *ctx, int P, const int32_t *d_order, in
   a.qcap = (uint32_t)std::min<int64_t>(room / 8, 4096);
   const size_t smem = sizeof(uint32_t) * ((size_t)a.vis_words + 2 * (size_t)a.qcap);
   const auto kernel = a.vis ? kcenters_block_kernel<false> : kcenters_block_kernel<true>;
-  PHDE_CK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int arc = phde_allow_smem(ctx, (const void *)kernel)) return arc;
   kernel<<<grid, KB_THREADS, smem, ctx->stream>>>(a);
   PHDE_LAUNCHED(ctx);
   return PHDE_OK;

@@ -521,7 +521,7 @@ int launch_scores(phde_ctx *ctx, const int32_t *d_d0, const ull *hop2, const uin
                   int64_t n, const float *wts, float *score, unsigned *hist, int nbins, const int32_t *gid) {
   if (getenv("PHDE_MLP_CUDA_CORES")) {
     const size_t mlp_smem = sizeof(float) * MLP_H * MLP_TILE + sizeof(unsigned) * nbins;
-    PHDE_CK(ctx, cudaFuncSetAttribute(mlp_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem));
+    if (int arc = phde_allow_smem(ctx, (const void *)mlp_score_kernel)) return arc;
     int gm = 0;
     if (int rc = mlp_grid(ctx, n, mlp_smem, &gm)) return rc;
     mlp_score_kernel<<<gm, 256, mlp_smem, ctx->stream>>>(ctx->d_off, d_d0, hop2, outw, maxes, n, wts, score, hist,
@@ -530,7 +530,7 @@ int launch_scores(phde_ctx *ctx, const int32_t *d_d0, const ull *hop2, const uin
     return PHDE_OK;
   }
   const size_t smem = TM_SMEM + sizeof(unsigned) * nbins;
-  PHDE_CK(ctx, cudaFuncSetAttribute(mlp_score_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int arc = phde_allow_smem(ctx, (const void *)mlp_score_tc_kernel)) return arc;
   // all of the unified L1/shared storage as shared memory: two CTAs of ~96 KB per SM
   PHDE_CK(ctx, cudaFuncSetAttribute(mlp_score_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                     (int)cudaSharedmemCarveoutMaxShared));

@@ -551,7 +551,7 @@ int phde_cgs2_mixed(phde_ctx *ctx, const int32_t *D, int P, const ull *sumsq, co
   const int64_t n = ctx->n;
   const size_t smem = sizeof(double) * (C2_THREADS / 32) * (size_t)(k + 2) + sizeof(float) * (C2_THREADS / 32) * 32 * TILE_LD;
   int per_sm = 0;
-  PHDE_CK(ctx, cudaFuncSetAttribute(cgs2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int arc = phde_allow_smem(ctx, (const void *)cgs2_kernel)) return arc;
   PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cgs2_kernel, C2_THREADS, smem));
   if (per_sm < 1) return phde_fail(ctx, PHDE_ERR_CUDA, "cgs2 kernel cannot be resident");
   per_sm = std::min(per_sm, 4);
@@ -668,9 +668,7 @@ int phde_coords_mixed(phde_ctx *ctx, const float *S, const double *Y, int k, int
   const int grid = grid_of(ctx, ctx->n, COORD_ROWS, 8);
   double *part = (double *)phde_buf(ctx, "coords32.part", sizeof(double) * grid * (size_t)COORD_MAXC);
   if (!part) return PHDE_ERR_OOM;
-  const size_t smem_max = sizeof(float) * ((size_t)COORD_ROWS * k + (size_t)k * COORD_MAXC);
-  PHDE_CK(ctx, cudaFuncSetAttribute(coords32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)std::max<size_t>(smem_max, 48 * 1024)));
+  if (int arc = phde_allow_smem(ctx, (const void *)coords32_kernel)) return arc;
   for (int t0 = 0; t0 < c; t0 += COORD_MAXC) {  // coordinates in groups of COORD_MAXC
     const int cg = std::min(COORD_MAXC, c - t0);
     const size_t smem = sizeof(float) * ((size_t)COORD_ROWS * k + (size_t)k * cg);

@@ -1010,7 +1010,7 @@ static int msbfs_run(phde_ctx *ctx, const int64_t *d_src, int nsrc, int nlist, i
     const char *we = getenv("PHDE_MSBFS_WINDOW");
     const bool win = we ? atoi(we) != 0 : ctx->ms_local;
     const size_t dyn = win ? sizeof(ull) * 3 * MS_WIN * W : 0;
-    PHDE_CK(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    if (int arc = phde_allow_smem(ctx, (const void *)fn)) return arc;
     // with a window, all of the unified L1/shared storage as shared memory (two CTAs per SM); without, the
     // default split
     PHDE_CK(ctx, cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -1147,7 +1147,7 @@ int phde_record_columns(phde_ctx *ctx, const uint16_t *R, int RW, const int *h_c
   PHDE_CK(ctx, cudaMemsetAsync(ssq, 0, sizeof(ull) * ncols, ctx->stream));
   PHDE_CK(ctx, cudaMemsetAsync(unr, 0, sizeof(int), ctx->stream));
   const size_t smem = sizeof(uint16_t) * 32 * (size_t)(RW + 2);
-  PHDE_CK(ctx, cudaFuncSetAttribute(gather_columns_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (int arc = phde_allow_smem(ctx, (const void *)gather_columns_kernel)) return arc;
   const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + 31) / 32, (int64_t)ctx->nsm * 4));
   gather_columns_kernel<<<g, 512, smem, ctx->stream>>>(R, n, RW, dcols, ncols, D, ssq, unr);
   PHDE_LAUNCHED(ctx);

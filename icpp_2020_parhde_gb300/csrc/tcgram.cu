@@ -293,11 +293,7 @@ template <int MT, int N, int OUT>
 int launch(phde_ctx *ctx, const TcGramArgs &a, dim3 grid) {
   constexpr int STAGE_BYTES = MT * A_TILE_BYTES + 3 * N * KC * 2;
   constexpr int SMEM = 2 * STAGE_BYTES;
-  static bool attr_set[64] = {};
-  if (!attr_set[ctx->device & 63]) {
-    PHDE_CK(ctx, cudaFuncSetAttribute(tc_gram_kernel<MT, N, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    attr_set[ctx->device & 63] = true;
-  }
+  if (int arc = phde_allow_smem(ctx, (const void *)tc_gram_kernel<MT, N, OUT>)) return arc;
   tc_gram_kernel<MT, N, OUT><<<grid, TC_THREADS, SMEM, ctx->stream>>>(a);
   PHDE_LAUNCHED(ctx);
   return PHDE_OK;
