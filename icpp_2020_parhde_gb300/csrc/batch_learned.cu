@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(BL_M) batch_fps_kernel(const int32_t *D, int64
 // (column, graph) into sumsq[(P0 + p) B + g], one atomic per warp when its 32 rows share a graph.
 __global__ void batch_record_cols_kernel(const uint16_t *R, int RW, int64_t N, const int32_t *gid, const int *ord,
                                          int P0, int P, int B, int32_t *D, ull *sumsq) {
-  extern __shared__ uint16_t tile[];  // [32][RW + 2]
+  extern __shared__ __align__(16) uint16_t tile[];  // [32][RW + 2]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int TLD = RW + 2, hw = RW / 2, Pn = P - P0;
   for (int64_t v0 = (int64_t)blockIdx.x * 32; v0 < N; v0 += (int64_t)gridDim.x * 32) {

@@ -70,7 +70,7 @@ __device__ __forceinline__ void stage_tile(const T *S, int64_t i0, int rows, int
 }
 
 __global__ void __launch_bounds__(CGS_THREADS) cgs_kernel(CgsArgs a) {
-  extern __shared__ double sm[];  // [nwarps][k+2] reduction scratch (coefficients in phase E), then tiles
+  extern __shared__ __align__(16) double sm[];  // [nwarps][k+2] reduction scratch (coefficients in phase E), then tiles
   __shared__ double red[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int64_t n = a.n;
@@ -614,7 +614,7 @@ __global__ void __launch_bounds__(256) gram_kernel(const double *A, const double
 template <int NO>
 __global__ void __launch_bounds__(1024) gram_list_kernel(const double *A, const double *B, int64_t n, int k,
                                                          double *part) {
-  extern __shared__ double gsm[];  // sA[GR][k + 1], sB[GR][k + 1]
+  extern __shared__ __align__(16) double gsm[];  // sA[GR][k + 1], sB[GR][k + 1]
   double *sA = gsm, *sB = gsm + GR * (k + 1);
   const int kp = k + 1;
   const int64_t rows_per = (n + gridDim.y - 1) / gridDim.y;
@@ -922,7 +922,7 @@ __device__ __forceinline__ void coords_row(const double *row, const double *Ys, 
 // count at compile time up to 3 (2 and 3 coordinates are what layouts ask for).
 __global__ void __launch_bounds__(128) coords_kernel(const double *M, const double *Y, int64_t n, int k, int c,
                                                      double *X, double *part) {
-  extern __shared__ double csm[];  // the group's Ys[q + t * k]
+  extern __shared__ __align__(16) double csm[];  // the group's Ys[q + t * k]
   __shared__ double red[32];
   const int rows = blockDim.x;
   double *Ys = csm;

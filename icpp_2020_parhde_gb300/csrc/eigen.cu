@@ -162,7 +162,7 @@ __global__ void __cluster_dims__(PW_CL, 1, 1) __launch_bounds__(EIG_THREADS)
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
-  extern __shared__ double psm[];
+  extern __shared__ __align__(16) double psm[];
   const int NO = (N + PW_CL - 1) / PW_CL;  // vectors owned per CTA
   double *Ks = psm;                         // N*N, column-major
   double *Eo = Ks + N * N;                  // NO*N: owned vector li at Eo + li*N
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(EIG_THREADS) jacobi_smem_kernel(const double *
 #define JS_MARK(i)                                              \
   if (trace && blockIdx.x == 0 && threadIdx.x == 0) trace[i] = global_timer_ns();
   JS_MARK(0)
-  extern __shared__ double js[];
+  extern __shared__ __align__(16) double js[];
   // a batch of problems: block b solves matrix b (N*N apart), with its own evals, sweeps and status
   Kin += (int64_t)blockIdx.x * N * N;
   K += (int64_t)blockIdx.x * N * N;

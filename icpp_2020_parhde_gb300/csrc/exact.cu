@@ -105,7 +105,7 @@ struct ZgArgs {
 // takes 80 registers, so four are resident.  8.0 M vertices, 76 columns: 11.1 -> 7.8 ms.
 __global__ void __launch_bounds__(ZG_THREADS, 3) zgram_kernel(ZgArgs a) {
   if (a.wide_only && __ldg(a.wide_only) <= 255u) return;  // uniform: the quad-layout kernel formed them
-  extern __shared__ int zsm[];  // [ZG_ROWS][S], zs4[ZG_ROWS/4][S], ys2[ZG_ROWS/2][S], then the record columns
+  extern __shared__ __align__(16) int zsm[];  // [ZG_ROWS][S], zs4[ZG_ROWS/4][S], ys2[ZG_ROWS/2][S], then the record columns
   __shared__ unsigned s_deg[ZG_ROWS], s_mz[ZG_THREADS / 32], s_md, s_sd;
   const int S = a.c1 + 4;
   uint32_t *zs4 = (uint32_t *)zsm + ZG_ROWS * S, *ys2 = zs4 + (ZG_ROWS / 4) * S;
@@ -769,7 +769,7 @@ struct CoefArgs {
 // reciprocals, the final sums) to one thread, broadcast through shared memory.
 __global__ void __launch_bounds__(CF_THREADS, 1) coef_kernel(CoefArgs a) {
   // rr[ld], gdr[ld], cq[k], rden[k], part[CF_THREADS], then (nc > 0) GIs[nc][nc], GDs[nc][nc], then (sa) As[k][ld]
-  extern __shared__ double cs[];
+  extern __shared__ __align__(16) double cs[];
   __shared__ int s_idx[PHDE_MAX_K];
   __shared__ double s_inv, s_c0, s_nrm;
   {  // out of the exact path's range (the host reads the same words and takes the FP64 vector kernels)
@@ -1037,7 +1037,7 @@ __global__ void __launch_bounds__(LG_THREADS, KP == 64 ? 4 : 2) lgram_kernel(LgA
   // instructions; T = sum z (x) s is accumulated and flushed doubled, self-loops (c z (x) z) go to T2 directly.
   // uint16 rows: zs[LG_ITEMS][SL], rs[LG_ITEMS][SL] as ints, u = 2 s + c z, one IMAD per item.
   constexpr bool PK = sizeof(T) == 1;
-  extern __shared__ int lsm[];
+  extern __shared__ __align__(16) int lsm[];
   __shared__ ull s_bnd[LG_ITEMS];
   __shared__ int s_self[LG_ITEMS];
   __shared__ int s_list[LG_ITEMS];  // phase 2 items of the slab
@@ -1499,7 +1499,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) coords_fix_kernel(const T *Z, int64_t n, int kp, int c, const int32_t *whi,
                                                          const uint32_t *wlo, const long long *w0fix,
                                                          const double *sinv, double *X, double *part) {
-  extern __shared__ uint32_t wsm[];  // per coordinate: hi[kp], lo[kp]
+  extern __shared__ __align__(16) uint32_t wsm[];  // per coordinate: hi[kp], lo[kp]
   __shared__ double red[32];
   for (int e = threadIdx.x; e < c * kp; e += blockDim.x) {
     wsm[2 * e] = (uint32_t)whi[e];

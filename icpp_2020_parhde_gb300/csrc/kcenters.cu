@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
   __shared__ unsigned s_listed;
   __shared__ uint32_t s_win[KC_THREADS / 32][32];
   __shared__ ull red[32];
-  extern __shared__ uint32_t s_hist[];  // [P]: every block keeps the same selection history; the list, the bitmap
+  extern __shared__ __align__(16) uint32_t s_hist[];  // [P]: every block keeps the same selection history; the list, the bitmap
   const KcList list{s_hist + ((a.P + 3) & ~3), &s_listed};
   uint32_t *s_bm = list.v + a.cap;
   const int full = a.cap / KC_THREADS - 1;  // iterations between looks at the list
@@ -505,7 +505,7 @@ constexpr int KB_THREADS = 1024;
 constexpr uint32_t KB_ROUND = 16;  // neighbours of a row per round: one round covers most rows of a geometric graph
 constexpr uint32_t KB_ROW = 256;  // neighbours of a row taken by its lane group; the rest by the whole warp
 
-extern __shared__ uint32_t kb_smem[];  // [vis_words] visited, then the two frontier lists
+extern __shared__ __align__(16) uint32_t kb_smem[];  // [vis_words] visited, then the two frontier lists
 
 struct KbLevel {
   const uint32_t *gq_in;  // frontier: entry i in kb_smem[s_in + i] below qcap, else in gq_in
@@ -873,7 +873,7 @@ __device__ __forceinline__ ull cluster_max(ull mine, ull *slots, uint32_t rank, 
 }
 
 __global__ void __launch_bounds__(KL_THREADS, 1) kcenters_cluster_kernel(KlArgs a) {
-  extern __shared__ uint32_t kl_smem[];  // list, visited, next[2], (row starts), history
+  extern __shared__ __align__(16) uint32_t kl_smem[];  // list, visited, next[2], (row starts), history
   __shared__ uint32_t s_counts[2][KL_MAX_CLUSTER];
   __shared__ ull s_keys[KL_MAX_CLUSTER], s_sums[KL_MAX_CLUSTER], s_fix[KL_MAX_CLUSTER];
   // of the two levels in turn: vertices listed, and whether a listed row is longer than KL_ROW

@@ -63,7 +63,7 @@ __device__ __forceinline__ void stage_tile32(const float *S, int64_t i0, int row
 }
 
 __global__ void __launch_bounds__(C2_THREADS) cgs2_kernel(Cgs2Args a) {
-  extern __shared__ double sm[];  // [nwarps][k+2] (coefficients as float in phase E), then float tiles
+  extern __shared__ __align__(16) double sm[];  // [nwarps][k+2] (coefficients as float in phase E), then float tiles
   __shared__ double red[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int64_t n = a.n;
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(256) sum_parts32_kernel(const double *part, in
 constexpr int COORD_ROWS = 128;
 __global__ void __launch_bounds__(COORD_ROWS) coords32_kernel(const float *S, const double *Y, int64_t n, int k, int c,
                                                               double *X, double *part) {
-  extern __shared__ float smc[];  // [COORD_ROWS * k] rows of S, then Ys[q * c + t]
+  extern __shared__ __align__(16) float smc[];  // [COORD_ROWS * k] rows of S, then Ys[q * c + t]
   __shared__ double red[32];
   float *rows = smc, *Ys = smc + COORD_ROWS * k;
   for (int idx = threadIdx.x; idx < k * c; idx += blockDim.x) {

@@ -823,7 +823,7 @@ __global__ void ms_heavy_plan_kernel(const int64_t *off, const uint32_t *adj, in
 // per-column exact sums of squares and an unreached flag on the way.
 __global__ void gather_columns_kernel(const uint16_t *R, int64_t n, int RW, const int *cols, int ncols, int32_t *D,
                                       ull *sumsq, int *unreached) {
-  extern __shared__ uint16_t tile[];  // [32][RW + 2]: the padded row stride puts consecutive rows in
+  extern __shared__ __align__(16) uint16_t tile[];  // [32][RW + 2]: the padded row stride puts consecutive rows in
                                       // consecutive banks (a plain 512-byte stride maps every lane to one bank)
   __shared__ ull s_ssq[GATHER_SMEM_COLS];  // per-CTA column sums; column p is always summed by warp p % nw
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
