@@ -1296,6 +1296,8 @@ int phde_run_bfs_batched_blocks(phde_ctx *ctx, int P, const int32_t *d_order, in
   PHDE_CK(ctx, cudaMemsetAsync(next, 0, sizeof(unsigned), ctx->stream));
   int rc = phde_fill_i32(ctx, min_d, N, 0x7fffffff);
   if (rc) return rc;
+  // the context's error word: what an earlier call left there, or a new context's memory, is not this call's
+  if ((rc = phde_reset_sync(ctx))) return rc;
   KbArgs a;
   a.off = ctx->d_off;
   a.adj = ctx->d_adj;

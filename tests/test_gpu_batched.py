@@ -227,3 +227,18 @@ def test_block_kcenters_row_list_and_bitmap_edges(monkeypatch, leaves):
     for rows in common:
         for a, b in zip(out["union"][rows], out["blocks"][rows]):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("mode", ["union", "blocks"])
+def test_batch_after_a_refused_batch(monkeypatch, mode):
+    """A batch with a graph that is not connected is refused, and the next batch on that context is not."""
+    monkeypatch.setenv("PHDE_BATCH_BFS", mode)
+    good = [graphs.mesh(20, 15, seed=i) for i in range(3)]
+    split = graphs._csr_from_undirected(40, np.delete(np.arange(39), 19), np.delete(np.arange(1, 40), 19))
+    with Context(0) as cb:
+        cb.upload_batch([good[0], split])
+        with pytest.raises(ParHDEError):
+            cb.layout_batched(4, 2)
+        cb.upload_batch(good)
+        xs, _ = cb.layout_batched(4, 2)
+        assert all(np.all(np.isfinite(x)) for x in xs)
