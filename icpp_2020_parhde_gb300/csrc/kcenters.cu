@@ -77,7 +77,7 @@ struct KcArgs {
   const int64_t *vbase;
   const int32_t *gid;
   ull *qinit;       // [1] level-0 queue counter of the pass (count << 32 | edges)
-  const int64_t *resume;  // passes kcenters_cluster_kernel finished, source of the next one (null: none)
+  const int64_t *resume;  // where kcenters_cluster_kernel stopped (KlArgs::resume; null: it did not run)
 };
 
 // Per-graph fold of a batched pass: the max of `key` and the sum of `ssq` over the lanes of one graph
@@ -157,10 +157,14 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
   uint32_t step = 0;
   ull edges_local = 0;
   int p0 = 0;
+  int32_t level0 = 0;  // levels of pass p0 that are done
+  int64_t edges0 = 0;  // and the edges that left them
   if (a.resume) {  // go on where the cluster stopped: the same history, from the passes' keys or sources
     p0 = (int)a.resume[0];
     if (p0 >= a.P) return;
     src = a.resume[1];
+    level0 = (int32_t)a.resume[2];
+    edges0 = a.resume[3];
     for (int i = tid; i < p0; i += blockDim.x)
       s_hist[i] = a.variant == 2 ? (uint32_t)a.sources[i] : 0xffffffffu - (uint32_t)(a.keys[i] & 0xffffffffull);
     __syncthreads();
@@ -171,7 +175,38 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
     int64_t s_off = 0;
     uint32_t sdeg = 0;
     uint32_t f_cnt = 1, f_edges = 0;
-    if (a.B == 0) {
+    const bool mid = p == p0 && level0 > 0;  // a pass that the cluster began
+    if (mid) {  // its last level, read back from the column, is the frontier (step is 0)
+      const bool once = n <= gstride;
+      int since = 0;
+      for (int64_t base = gbase; base < n; base += gstride) {
+        const int64_t v = base + tid;
+        const bool f = v < n && Dp[v] == level0;
+        const uint32_t bal = __ballot_sync(PHDE_FULL_MASK, f);
+        const int64_t v0 = v - (tid & 31);
+        if ((tid & 31) == 0 && v0 < n) a.bm[0][v0 >> 5] = bal;
+        if (once) {
+          uint32_t ov = 0, dv = 0;
+          if (f) {
+            ov = (uint32_t)__ldg(a.off + v);
+            dv = (uint32_t)__ldg(a.off + v + 1) - ov;
+          }
+          block_push(f, (uint32_t)v, dv, a.qv0, a.qe0, a.qinit, &psc, a.qo0, ov);
+          break;
+        }
+        list.add(f, (uint32_t)v);
+        if (++since == full) {
+          since = 0;
+          __syncthreads();
+          if (__syncthreads_or(s_listed > KC_THREADS)) list.flush(a.off, a.qv0, a.qe0, a.qo0, a.qinit, &psc);
+        }
+      }
+      if (!once) list.flush(a.off, a.qv0, a.qe0, a.qo0, a.qinit, &psc);
+      ull q;
+      if (!grid_sync_read(a.gs, a.err, a.timeout_ns, a.qinit, &q)) return;
+      f_cnt = (uint32_t)(q >> 32);
+      f_edges = (uint32_t)(q & 0xffffffffull);
+    } else if (a.B == 0) {
       if (tid == 0) {
         Dp[src] = 0;
         // the level-0 frontier bitmap holds only the source (the previous pass left it empty)
@@ -211,10 +246,10 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
       f_cnt = (uint32_t)(q >> 32);
       f_edges = (uint32_t)(q & 0xffffffffull);
     }
-    int64_t edges_to_check = a.nnz, scout = f_edges;
+    int64_t edges_to_check = mid ? a.nnz - edges0 : a.nnz, scout = f_edges;
     bool in_bu = false;
     int64_t awake = 0, old_awake = 0;
-    int32_t L = 0;
+    int32_t L = mid ? level0 : 0;
 
     while (f_cnt > 0) {
       if (!in_bu) {
@@ -750,7 +785,8 @@ __global__ void __launch_bounds__(KB_THREADS) kcenters_block_kernel(KbArgs a) {
 //   scan     the owner takes next & ~visited of its words: new vertices, their distances and its next list.
 // Only the adjacency is read from L2.  Every CTA posts its frontier's size to all others before the barrier, so all
 // see the same total: 0 ends the pass, more than `limit` (a wide level: the whole grid is faster) leaves the
-// kernel, and kcenters_bfs_kernel, launched after it, goes on from the pass that was not finished.
+// kernel, and kcenters_bfs_kernel, launched after it, goes on from that level: it reads the level's vertices back from
+// the distance column.
 // Sources, history and duplicate fix-up as in kcenters_bfs_kernel; distances are unique, so the results are equal.
 // Measured (16 CTAs of 512 threads): a level was 3100 clocks on the 125 x 125 mesh (expand 840, barrier with the ORs in
 // flight 1240, scan 990) and 4000 on a 150k-vertex 2-D geometric graph before the words were dealt to the scanning
@@ -767,7 +803,9 @@ struct KlArgs {
   int32_t *min_d;
   ull *sumsq, *keys, *edges;
   int *err;
-  int64_t *resume;   // [2]: passes finished, source of the next one
+  // [5]: passes finished; of the next one its source, the level it stopped at (0: not begun) and the edges of the
+  // levels before that; 0, the counter of the queue that kcenters_bfs_kernel makes of that level
+  int64_t *resume;
   int words;         // words owned by a CTA
   int rows;          // row starts in shared memory
   uint32_t limit;
@@ -904,6 +942,7 @@ __global__ void __launch_bounds__(KL_THREADS, 1) kcenters_cluster_kernel(KlArgs 
   uint32_t edges = 0;
   ull edges_all = 0;
   int64_t src = a.variant == 1 ? a.fixed_src[0] : 0;
+  if (tid == 0 && rank == 0) a.resume[3] = a.resume[4] = 0;
   for (int p = 0; p < a.P; p++) {
     int32_t *Dp = a.D + (int64_t)p * a.n;
     for (int w = tid; w < 3 * words; w += KL_THREADS) vis[w] = 0u;
@@ -919,10 +958,11 @@ __global__ void __launch_bounds__(KL_THREADS, 1) kcenters_cluster_kernel(KlArgs 
     if (tid == 0 && rank == 0) a.sources[p] = src;
     cluster_barrier();  // every CTA's words are clear
     l.cnt = mine ? 1u : 0u;
-    uint32_t L = 0;
+    uint32_t L = 0, before = 0;  // before: `edges` of the levels before L
     bool wide = false;
     for (;;) {
       const uint32_t par = L & 1;
+      before = edges;
       l.next = next_s + par * 4u * words;
       // ---- expand ----
       if (tid == 0) {  // for the scan after the barrier; what the last scan left is in the other place
@@ -993,19 +1033,18 @@ __global__ void __launch_bounds__(KL_THREADS, 1) kcenters_cluster_kernel(KlArgs 
       __syncthreads();
       l.cnt = *(volatile uint32_t *)&s_cnt[par];
     }
-    edges_all += edges;
-    edges = 0;
-    if (wide) {  // leave the pass to the whole grid: its column as it was, the source to start from
-      for (int i = tid; i < 32 * words; i += KL_THREADS) {
-        const int64_t v = ((((int64_t)(i >> 5) << l.clog) | rank) << 5) | (i & 31);
-        if (v < a.n) Dp[v] = -1;
-      }
+    edges_all += before;  // of a finished pass all: its last level found nothing
+    if (wide) {  // leave the rest of the pass to the whole grid, which expands level L again
+      const ull e = block_sum((ull)before, red);
+      if (tid == 0) atomicAdd((ull *)a.resume + 3, e);
       if (tid == 0 && rank == 0) {
         a.resume[0] = p;
         a.resume[1] = src;
+        a.resume[2] = L;
       }
       break;
     }
+    edges = 0;
     // ---- fold the CTA's vertices: min distance, farthest vertex, sum of squares ----
     ull kbest = 0, ssq = 0;
     int bad = 0;
@@ -1053,6 +1092,7 @@ __global__ void __launch_bounds__(KL_THREADS, 1) kcenters_cluster_kernel(KlArgs 
       a.sumsq[p] = s;
       a.keys[p] = key;
       a.resume[0] = p + 1;
+      a.resume[2] = 0;
     }
     if (p + 1 == a.P) break;
     if (a.variant == 1) {
@@ -1102,11 +1142,11 @@ int phde_fill_i32(phde_ctx *ctx, int32_t *p, int64_t n, int32_t v) {
 }
 
 // The passes on one cluster first, where the graph may have narrow levels and its bitmaps fit the cluster's shared
-// memory; *resume tells the whole-grid kernel what is left.  Average degree above KL_DEGREE: scale-free graphs,
+// memory; g.resume tells the whole-grid kernel what is left.  Average degree above KL_DEGREE: scale-free graphs,
 // whose second or third level is most of the graph.
 constexpr int64_t KL_DEGREE = 24;
 
-static int run_cluster_passes(phde_ctx *ctx, const KcArgs &g, const int64_t **resume) {
+static int run_cluster_passes(phde_ctx *ctx, KcArgs &g) {
   if (g.nnz > KL_DEGREE * g.n) return PHDE_OK;
   const auto kernel = kcenters_cluster_kernel;
   int C = KL_MAX_CLUSTER;
@@ -1137,7 +1177,7 @@ static int run_cluster_passes(phde_ctx *ctx, const KcArgs &g, const int64_t **re
     if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit >= 1) break;
     cudaGetLastError();
   }
-  int64_t *res = (int64_t *)phde_buf(ctx, "kl.resume", sizeof(int64_t) * 2);
+  int64_t *res = (int64_t *)phde_buf(ctx, "kl.resume", sizeof(int64_t) * 5);
   if (!res) return PHDE_ERR_OOM;
   a.off = g.off;
   a.adj = g.adj;
@@ -1157,7 +1197,8 @@ static int run_cluster_passes(phde_ctx *ctx, const KcArgs &g, const int64_t **re
   a.limit = KL_LIST;
   PHDE_CK(ctx, cudaLaunchKernelEx(&cfg, kernel, a));
   PHDE_LAUNCHED(ctx);
-  *resume = res;
+  g.resume = res;
+  g.qinit = (ull *)(res + 4);
   return PHDE_OK;
 }
 
@@ -1262,7 +1303,7 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   cudaEventRecord(ctx->kev[0], ctx->stream);
   a.resume = nullptr;
   // a traced call keeps every pass in the kernel that writes the timeline
-  if (B == 0 && !a.trace && (rc = run_cluster_passes(ctx, a, &a.resume))) return rc;
+  if (B == 0 && !a.trace && (rc = run_cluster_passes(ctx, a))) return rc;
   PHDE_CK(ctx, cudaLaunchCooperativeKernel((const void *)kcenters_bfs_kernel, dim3(ctx->nsm * per_sm),
                                            dim3(KC_THREADS), args, smem, ctx->stream));
   PHDE_LAUNCHED(ctx);

@@ -279,3 +279,31 @@ def test_kcenters_levels_of_one_and_more_grid_iterations(gpu_ctx, make):
     D, s = gpu_ctx.kcenters(4, 0)
     Do, so = orc.kcenters(g, 4, 0, parallel=True)
     assert np.array_equal(s, so) and np.array_equal(D, Do)
+
+
+def _hub_mesh(nx: int, ny: int, leaves: int):
+    """A mesh whose last vertex carries `leaves` leaves: narrow levels, then one wide one."""
+    g = graphs.mesh(nx, ny, seed=31)
+    src = np.repeat(np.arange(g.n), np.diff(g.offsets.astype(np.int64)))
+    keep = src < g.adj
+    lo = np.concatenate([src[keep], np.full(leaves, g.n - 1)])
+    hi = np.concatenate([g.adj[keep].astype(np.int64), g.n + np.arange(leaves)])
+    return graphs._csr_from_undirected(g.n + leaves, lo, hi)
+
+
+@pytest.mark.parametrize("nx,ny,leaves", [(100, 100, 5000), (37, 20, 4097), (500, 400, 30000), (100, 100, 250_000)])
+def test_wide_level_continues_on_the_grid(gpu_ctx, nx, ny, leaves):
+    """A level too wide for the cluster goes on from there on the whole grid: the oracle's distances, from sources
+    before, at and behind the wide level, and the levels before it are not searched again."""
+    g = _hub_mesh(nx, ny, leaves)
+    gpu_ctx.upload(g)
+    for s in (0, nx * ny - 1, g.n - 1):
+        assert np.array_equal(gpu_ctx.distances([s])[:, 0], orc.bfs(g, s))
+    D, src = gpu_ctx.kcenters(5, 0)
+    Do, so = orc.kcenters(g, 5, 0, parallel=True)
+    assert np.array_equal(src, so) and np.array_equal(D, Do)
+    if leaves * 6 < g.nnz:  # the hub's level is no bottom-up step
+        # the first pass crosses the mesh before the hub: begun again, it would add the mesh's entries (over 0.8 nnz).
+        # A bottom-up level may read a row that the next reads again, at most in the last levels: half a pass is left.
+        r = gpu_ctx.layout("ParHDE", "Kcenters", k=2, c=2)
+        assert 0 < r.stats["edges_examined"] <= 6.5 * g.nnz
