@@ -1143,11 +1143,17 @@ int phde_fill_i32(phde_ctx *ctx, int32_t *p, int64_t n, int32_t v) {
 
 // The passes on one cluster first, where the graph may have narrow levels and its bitmaps fit the cluster's shared
 // memory; g.resume tells the whole-grid kernel what is left.  Average degree above KL_DEGREE: scale-free graphs,
-// whose second or third level is most of the graph.
+// whose second or third level is most of the graph.  More than KL_VERTICES: every level scans the CTAs' words, whose
+// number grows with the graph, and the grid alone is as fast from 4 million on (four passes, grid alone against cluster:
+// meshes of 1.0, 2.0, 2.9, 4.0 and 5.8 million vertices 25.8 / 15.0, 37.4 / 27.7, 47.9 / 41.2, 56.9 / 55.5 and
+// 69.7 / 84.9 ms; one source in the middle of the 4-million mesh 12.4 / 13.7, of 3 million in 2-D 9.7 / 9.6).
+// The width at which a pass moves to the grid is the list's size: smaller ones were never faster up to a million vertices
+// (12 passes at 1024, 2048, 3072 and 4096: 60k in 3-D 3.73, 3.71, 2.58, 2.58 ms; 60^3 grid 9.97, 9.95, 8.98, 5.55).
 constexpr int64_t KL_DEGREE = 24;
+constexpr int64_t KL_VERTICES = (int64_t)3 << 20;
 
 static int run_cluster_passes(phde_ctx *ctx, KcArgs &g) {
-  if (g.nnz > KL_DEGREE * g.n) return PHDE_OK;
+  if (g.nnz > KL_DEGREE * g.n || g.n > KL_VERTICES) return PHDE_OK;
   const auto kernel = kcenters_cluster_kernel;
   int C = KL_MAX_CLUSTER;
   KlArgs a;

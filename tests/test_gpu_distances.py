@@ -307,3 +307,18 @@ def test_wide_level_continues_on_the_grid(gpu_ctx, nx, ny, leaves):
         # A bottom-up level may read a row that the next reads again, at most in the last levels: half a pass is left.
         r = gpu_ctx.layout("ParHDE", "Kcenters", k=2, c=2)
         assert 0 < r.stats["edges_examined"] <= 6.5 * g.nnz
+
+
+@pytest.mark.parametrize("ny", [1536, 1537], ids=["3<<20", "past it"])
+def test_cluster_size_limit(gpu_ctx, ny):
+    """Meshes of the most vertices the cluster takes and of more, which stay on the grid."""
+    g = graphs.mesh(2048, ny, seed=33)
+    gpu_ctx.upload(g)
+    before = gpu_ctx.launch_count
+    D, s = gpu_ctx.kcenters(2, 0)
+    launches = gpu_ctx.launch_count - before
+    Do, so = orc.kcenters(g, 2, 0, parallel=True)
+    assert np.array_equal(s, so) and np.array_equal(D, Do)
+    before = gpu_ctx.launch_count
+    gpu_ctx.kcenters(2, 0)
+    assert gpu_ctx.launch_count - before == launches == (3 if g.n == 3 << 20 else 2)  # fill, (cluster), grid
