@@ -52,16 +52,22 @@ __global__ void widen_offsets_kernel(const uint32_t *in, int64_t *out, int64_t c
     out[i] = (int64_t)in[i];
 }
 
-// Device-side CSR validation: offsets start at 0, never decrease, end at nnz; neighbours < n.
-__global__ void validate_csr_kernel(const int64_t *off, const uint32_t *adj, int64_t n, int64_t nnz, int *bad) {
+// Device-side CSR validation: offsets start at 0, never decrease, end at nnz; neighbours < n.  bad[0]: a fault;
+// bad[1]: the largest degree.
+__global__ void validate_csr_kernel(const int64_t *off, const uint32_t *adj, int64_t n, int64_t nnz, unsigned *bad) {
   int b = 0;
+  unsigned most = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    if (off[i + 1] < off[i]) b = 1;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const int64_t d = off[i + 1] - off[i];
+    if (d < 0) b = 1;
+    most = (unsigned)d > most ? (unsigned)d : most;
+  }
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += stride)
     if ((int64_t)adj[e] >= n) b = 1;
   if (blockIdx.x == 0 && threadIdx.x == 0 && (off[0] != 0 || off[n] != nnz)) b = 1;
-  if (b) atomicExch(bad, 1);
+  if (b) atomicExch(bad, 1u);
+  block_atomic_max_u32(most, bad + 1);
 }
 
 // A barrier that waits for one more block than is launched: the bounded wait must give up.
@@ -297,20 +303,22 @@ int phde_graph_upload(phde_ctx *ctx, const void *offsets, int offset_bytes, cons
     if (nnz > 0)
       PHDE_CK(ctx, cudaMemcpyAsync(ctx->d_w, weights, sizeof(int32_t) * nnz, cudaMemcpyHostToDevice, ctx->stream));
   }
-  int *bad = (int *)phde_buf(ctx, "upload.bad", sizeof(int));
+  unsigned *bad = (unsigned *)phde_buf(ctx, "upload.bad", sizeof(unsigned) * 2);
   if (!bad) return PHDE_ERR_OOM;
-  PHDE_CK(ctx, cudaMemsetAsync(bad, 0, sizeof(int), ctx->stream));
+  PHDE_CK(ctx, cudaMemsetAsync(bad, 0, sizeof(unsigned) * 2, ctx->stream));
   validate_csr_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>((std::max(n, nnz) + 255) / 256, ctx->nsm * 8)), 256, 0,
                         ctx->stream>>>(ctx->d_off, ctx->d_adj, n, nnz, bad);
   PHDE_LAUNCHED(ctx);
-  int h = 0;
-  PHDE_CK(ctx, cudaMemcpyAsync(&h, bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  unsigned h[2] = {0, 0};
+  PHDE_CK(ctx, cudaMemcpyAsync(h, bad, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
   PHDE_CK(ctx, cudaStreamSynchronize(ctx->stream));
-  if (h) {
+  if (h[0]) {
     ctx->n = ctx->nnz = 0;
     return phde_fail(ctx, PHDE_ERR_CSR, "phde_graph_upload: offsets must start at 0, never decrease and end at nnz; "
                                         "neighbours must be < n");
   }
+  ctx->max_degree = h[1];
+  ctx->max_degree_epoch = ctx->graph_epoch;
   return PHDE_OK;
 }
 

@@ -206,6 +206,17 @@ __device__ __forceinline__ ull block_max_u64(ull v, ull *scratch) {
   return r;
 }
 
+// *out = max(*out, every thread's v), one atomic per block.  Called by all its threads.
+__device__ __forceinline__ void block_atomic_max_u32(unsigned v, unsigned *out) {
+  __shared__ unsigned s_max;
+  if (threadIdx.x == 0) s_max = 0u;
+  __syncthreads();
+  v = warp_max_u32(v);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_max, v);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_max) atomicMax(out, s_max);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Block-aggregated append to a frontier queue.  Each flagged thread appends vertex v with out-degree
 // dv.  One 64-bit atomic per block advances both the slot count (high 32 bits) and the running edge

@@ -47,8 +47,9 @@ struct phde_ctx {
   int64_t ws_epoch = 0;                            // bumped whenever a workspace buffer is (re)allocated
   // SSSP band width: the mean edge weight of the uploaded graph (sssp.cu)
   double w_mean = 1.0;
-  int64_t w_maxdeg = 0;  // and the largest degree, which picks the kernel
   long long w_mean_epoch = -1;
+  unsigned max_degree = 0;  // of the uploaded graph, found when it was checked or converted: picks the SSSP kernel
+  long long max_degree_epoch = -1;
   int eig_start = 0;               // start-vector values of the power iteration held by eig_start_buf (eigen.cu)
   const void *eig_start_buf = nullptr;
   // drawing (draw.cu): the entry-row array's graph, and the size of the last image drawn

@@ -122,9 +122,14 @@ __global__ void mtx_keep_kernel(const uint32_t *parent, int64_t n, const ull *be
     keep[v] = parent[v] == root ? 1u : 0u;
 }
 __global__ void mtx_newdeg_kernel(const uint32_t *keep, const uint32_t *newid, const int64_t *deg, int64_t n,
-                                  int64_t *ndeg) {
+                                  int64_t *ndeg, unsigned *maxdeg) {
+  unsigned most = 0;
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
-    if (keep[v]) ndeg[newid[v]] = deg[v];
+    if (keep[v]) {
+      ndeg[newid[v]] = deg[v];
+      most = (unsigned)deg[v] > most ? (unsigned)deg[v] : most;
+    }
+  block_atomic_max_u32(most, maxdeg);
 }
 __global__ void mtx_place_kernel(const ull *ukey, const int32_t *uw, int64_t E, const int64_t *rowstart,
                                  const uint32_t *keep, const uint32_t *newid, const int64_t *noff, uint32_t *adj,
@@ -279,7 +284,7 @@ extern "C" int phde_graph_from_entries(phde_ctx *ctx, const uint32_t *u, const u
   const int64_t Nn = hn;
   // ---- the kept component: new offsets, edges at their row positions ----
   PHDE_CK(ctx, cudaMemsetAsync(ndeg, 0, sizeof(int64_t) * (N + 1), ctx->stream));
-  mtx_newdeg_kernel<<<grid_for(ctx, N), 256, 0, ctx->stream>>>(keep, newid, deg, N, ndeg);
+  mtx_newdeg_kernel<<<grid_for(ctx, N), 256, 0, ctx->stream>>>(keep, newid, deg, N, ndeg, (unsigned *)bad + 2);
   PHDE_LAUNCHED(ctx);
   if (Nn + 1 > ctx->off_cap || !ctx->d_off) {
     cudaFree(ctx->d_off);
@@ -294,7 +299,9 @@ extern "C" int phde_graph_from_entries(phde_ctx *ctx, const uint32_t *u, const u
   if (!tmp4) return PHDE_ERR_OOM;
   PHDE_CK(ctx, cub::DeviceScan::ExclusiveSum(tmp4, t6, ndeg, ctx->d_off, Nn + 1, ctx->stream));
   int64_t nnz = 0;
+  unsigned maxdeg = 0;
   PHDE_CK(ctx, cudaMemcpyAsync(&nnz, ctx->d_off + Nn, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+  PHDE_CK(ctx, cudaMemcpyAsync(&maxdeg, bad + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
   PHDE_CK(ctx, cudaStreamSynchronize(ctx->stream));
   if (nnz > ctx->adj_cap || !ctx->d_adj) {
     cudaFree(ctx->d_adj);
@@ -317,6 +324,8 @@ extern "C" int phde_graph_from_entries(phde_ctx *ctx, const uint32_t *u, const u
   ctx->weighted = w != nullptr;
   ctx->batch_B = 0;
   ctx->graph_epoch++;
+  ctx->max_degree = maxdeg;
+  ctx->max_degree_epoch = ctx->graph_epoch;
   if (info) {
     info->n_in = N;
     info->nnz_dedup = E;

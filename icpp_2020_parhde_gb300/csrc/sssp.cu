@@ -553,21 +553,13 @@ __global__ void select_kernel(const ull *key_in, const int32_t *min_d, int64_t n
 int phde_fill_i32(phde_ctx *ctx, int32_t *p, int64_t n, int32_t v);
 
 namespace {
-// sum of the (non-negative) edge weights, for the band width, and the largest degree
-__global__ void weight_stats_kernel(const int64_t *off, const int32_t *w, int64_t n, int64_t nnz, ull *out) {
-  ull s = 0, m = 0;
+// sum of the (non-negative) edge weights, for the band width
+__global__ void weight_sum_kernel(const int32_t *w, int64_t nnz, ull *sum) {
+  ull s = 0;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += (int64_t)gridDim.x * blockDim.x)
     s += (ull)(w[e] > 0 ? w[e] : 0);
-  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-    const ull d = (ull)(off[v + 1] - off[v]);
-    m = d > m ? d : m;
-  }
   s = warp_sum(s);
-  m = warp_max_u64(m);
-  if ((threadIdx.x & 31) == 0) {
-    if (s) atomicAdd(out, s);
-    atomicMax(out + 1, m);
-  }
+  if ((threadIdx.x & 31) == 0 && s) atomicAdd(sum, s);
 }
 }  // namespace
 
@@ -581,30 +573,29 @@ int phde_run_sssp(phde_ctx *ctx, const int64_t *d_src, int32_t *d_col, int32_t d
   // a 256^3 grid with weights in [1, 255] a band of 8 mean weights is three times faster (on a 64^3 grid,
   // where every round is short, the wide band is as fast or faster).  So graphs of 2^20 vertices or more
   // use min(delta, max(64, 8 * mean weight)); PHDE_SSSP_DELTA sets the band outright.
-  if (ctx->w_mean_epoch != ctx->graph_epoch) {
-    ull *wstat = (ull *)phde_buf(ctx, "ss.wstat", 2 * sizeof(ull));
-    if (!wstat) return PHDE_ERR_OOM;
-    PHDE_CK(ctx, cudaMemsetAsync(wstat, 0, 2 * sizeof(ull), ctx->stream));
-    const int g = (int)std::max<int64_t>(1, std::min<int64_t>((std::max(ctx->nnz, n) + 255) / 256, (int64_t)ctx->nsm * 8));
-    weight_stats_kernel<<<g, 256, 0, ctx->stream>>>(ctx->d_off, ctx->d_w, n, ctx->nnz, wstat);
-    PHDE_LAUNCHED(ctx);
-    ull h[2] = {0, 0};
-    PHDE_CK(ctx, cudaMemcpyAsync(h, wstat, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    PHDE_CK(ctx, cudaStreamSynchronize(ctx->stream));
-    ctx->w_mean = ctx->nnz > 0 ? (double)h[0] / (double)ctx->nnz : 1.0;
-    ctx->w_maxdeg = (int64_t)h[1];
-    ctx->w_mean_epoch = ctx->graph_epoch;
-  }
   if (const char *e = getenv("PHDE_SSSP_DELTA")) {
     delta = atoi(e);
   } else if (n >= (int64_t)1 << 20) {
+    if (ctx->w_mean_epoch != ctx->graph_epoch) {
+      ull *wsum = (ull *)phde_buf(ctx, "ss.wsum", sizeof(ull));
+      if (!wsum) return PHDE_ERR_OOM;
+      PHDE_CK(ctx, cudaMemsetAsync(wsum, 0, sizeof(ull), ctx->stream));
+      const int g = (int)std::max<int64_t>(1, std::min<int64_t>((ctx->nnz + 255) / 256, (int64_t)ctx->nsm * 8));
+      weight_sum_kernel<<<g, 256, 0, ctx->stream>>>(ctx->d_w, ctx->nnz, wsum);
+      PHDE_LAUNCHED(ctx);
+      ull h = 0;
+      PHDE_CK(ctx, cudaMemcpyAsync(&h, wsum, sizeof(ull), cudaMemcpyDeviceToHost, ctx->stream));
+      PHDE_CK(ctx, cudaStreamSynchronize(ctx->stream));
+      ctx->w_mean = ctx->nnz > 0 ? (double)h / (double)ctx->nnz : 1.0;
+      ctx->w_mean_epoch = ctx->graph_epoch;
+    }
     const double band = std::max(64.0, 8.0 * ctx->w_mean);
     if (band < (double)delta) delta = (int32_t)band;
   }
   if (delta < 1) delta = 1;
   const char *le = getenv("PHDE_SSSP_LOCAL");
   const int lmax = le ? std::max(0, atoi(le)) : 0;
-  const bool group = lmax == 0 && ctx->w_maxdeg <= SG_MAX_ROW;
+  const bool group = lmax == 0 && ctx->max_degree_epoch == ctx->graph_epoch && ctx->max_degree <= SG_MAX_ROW;
   uint32_t *qv0, *qv1, *qe0 = nullptr, *qe1 = nullptr, *qo0 = nullptr, *qo1 = nullptr;
   if (group) {
     qv0 = (uint32_t *)phde_buf(ctx, "ss.q0", sizeof(uint4) * n);
@@ -644,7 +635,7 @@ int phde_run_sssp(phde_ctx *ctx, const int64_t *d_src, int32_t *d_col, int32_t d
   const int want = ce ? (atoi(ce) == 1 ? 1 : 2) : (n < ((int64_t)1 << (group ? 18 : 20)) ? 1 : 2);
   const void *kfn = want == 1 ? (const void *)sssp_nearfar_kernel<1> : (const void *)sssp_nearfar_kernel<2>;
   if (group) {  // (lanes, edges per lane) by the longest row
-    const int shape = ctx->w_maxdeg <= 8 ? 0 : ctx->w_maxdeg <= 16 ? 1 : 2;
+    const int shape = ctx->max_degree <= 8 ? 0 : ctx->max_degree <= 16 ? 1 : 2;
     static const void *const kernels[3][2] = {
         {(const void *)sssp_group_kernel<8, 1, 1>, (const void *)sssp_group_kernel<8, 1, 2>},
         {(const void *)sssp_group_kernel<16, 1, 1>, (const void *)sssp_group_kernel<16, 1, 2>},

@@ -322,3 +322,28 @@ def test_cluster_size_limit(gpu_ctx, ny):
     before = gpu_ctx.launch_count
     gpu_ctx.kcenters(2, 0)
     assert gpu_ctx.launch_count - before == launches == (3 if g.n == 3 << 20 else 2)  # fill, (cluster), grid
+
+
+@pytest.mark.parametrize("make", [lambda: graphs.rmat(11, seed=5), lambda: graphs.mesh(30, 20, seed=6)],
+                         ids=["edge-balanced", "lane-groups"])
+def test_sssp_first_search_on_a_graph_launches_no_more_than_the_next(gpu_ctx, make):
+    """The kernel is picked by what the upload found: no pass over the graph and no wait before a graph's first search
+    (below 2^20 vertices, where the band does not depend on the weights)."""
+    g = graphs.with_random_weights(make(), seed=3)
+    gpu_ctx.upload(g)
+    counts = []
+    for _ in range(2):
+        before = gpu_ctx.launch_count
+        assert np.array_equal(gpu_ctx.distances([1])[:, 0], orc.sssp(g, 1))
+        counts.append(gpu_ctx.launch_count - before)
+    assert counts[0] == counts[1]
+
+
+@pytest.mark.parametrize("hub", [32, 33])
+def test_sssp_on_a_converted_graph(gpu_ctx, hub):
+    """The largest degree is known for graphs made from matrix entries as well."""
+    g = graphs.with_random_weights(_two_stars(hub - 1, 5), seed=4)
+    src = np.repeat(np.arange(g.n), np.diff(g.offsets.astype(np.int64)))
+    low = src > g.adj
+    gpu_ctx.graph_from_entries(src[low] + 1, g.adj[low] + 1, g.weights[low], g.n, g.n, True)
+    assert np.array_equal(gpu_ctx.distances([3])[:, 0], orc.sssp(g, 3))
