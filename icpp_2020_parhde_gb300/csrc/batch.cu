@@ -16,8 +16,8 @@
 //   coordinates   X_b = S_b Y_b per segment, FP64 column norms per graph.
 // Nothing between the Kcenters launch and the coordinate copy waits on the host, so after the first call
 // the whole sequence is captured once into a CUDA graph and replayed.  The segment length (rows per CTA) is
-// picked by a small autotuner: the dense stages are timed at each candidate length on the caller's own batch at
-// the first call (the distances do not depend on it).
+// picked by a small autotuner: the dense stages are timed at increasing lengths on the caller's own batch at the first
+// call (the distances do not depend on it) until a longer one no longer gains.
 // Options outside that pipeline (FP64 or exact arithmetic, k above 32, the power iteration, the other
 // algorithms) lay the graphs out one after another with the single-graph pipeline (layout_per_graph): each
 // graph's CSR is cut out of the union on the device and laid out as if uploaded alone.
@@ -835,39 +835,50 @@ extern "C" int phde_layout_batched(phde_ctx *ctx, const phde_layout_opts *o, dou
     return PHDE_OK;
   };
   int rc;
-  // the tuned length is kept for batches of the same shape (count, vertices, entries, k); the captured
-  // graph is rebuilt after every upload (the device CSR may have moved)
-  const int64_t shape = ((int64_t)B * 1000003 + N) * 1000003 + ctx->nnz;
-  const bool tune = ctx->batch_tuned_shape != shape || ctx->batch_tuned_k != k;
+  // the tuned length is kept for batches of the same graph sizes (an FNV-1a hash of their vertices and entries), k and
+  // c; the captured graph is rebuilt after every upload (the device CSR may have moved)
+  uint64_t sizes = 14695981039346656037ull;
+  for (const std::vector<int64_t> *base : {&ctx->batch_vbase, &ctx->batch_ebase})
+    for (int64_t x : *base) sizes = (sizes ^ (uint64_t)x) * 1099511628211ull;
+  const bool tune = ctx->batch_tuned_sizes != sizes || ctx->batch_tuned_k != k || ctx->batch_tuned_c != c;
   if (ctx->batch_graph && ctx->batch_graph_epoch != ctx->graph_epoch) {
     cudaGraphExecDestroy(ctx->batch_graph);
     ctx->batch_graph = nullptr;
   }
+  int64_t dist_launches = 0;  // of the distances, where the tuning needs them before the timed run
   if (tune) {
-    // Only the stages on segments depend on the length, so the distance columns are computed once and each
-    // candidate is timed on those stages; a longer segment has to be 3 % faster than the best shorter one, which
-    // is more than their times vary, so that a batch is laid out with the same partial sums every time.
+    // Only the stages on segments depend on the length: the distance columns are computed once, and the lengths tried in
+    // increasing order (the dense stages' median of three runs) until one is not 3 % faster than the best before it.
+    // It is a measurement: where two lengths differ by about that much, two calls can pick differently and their partial
+    // sums round differently; at one length a batch's layouts are the same bits every time.
     static const int64_t kCandidates[] = {2048, 4096, 8192, 16384, 32768};
     float best = 1e30f;
     int64_t best_rows = kCandidates[0];
+    dist_launches = -ctx->launches;
+    cudaEventRecord(ctx->ev[4], ctx->stream);
     if ((rc = batch_distances(ctx, q, k))) return rc;
+    cudaEventRecord(ctx->ev[5], ctx->stream);
+    dist_launches += ctx->launches;
     if ((rc = set_segments(kCandidates[0])) || (rc = batch_dense(ctx, q, k, c))) return rc;  // untimed: first launches
     for (int64_t rows : kCandidates) {
       if ((rc = set_segments(rows))) return rc;
-      cudaEventRecord(ctx->ev[0], ctx->stream);
-      if ((rc = batch_dense(ctx, q, k, c))) return rc;
-      cudaEventRecord(ctx->ev[1], ctx->stream);
-      if ((rc = phde_check_device_err(ctx, "batched layout (tuning)"))) return rc;
-      float ms = 0;
-      cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
-      if (ms < 0.97f * best) {
-        best = ms;
-        best_rows = rows;
+      float t[3] = {0, 0, 0};
+      for (float &ms : t) {
+        cudaEventRecord(ctx->ev[2], ctx->stream);
+        if ((rc = batch_dense(ctx, q, k, c))) return rc;
+        cudaEventRecord(ctx->ev[3], ctx->stream);
+        if ((rc = phde_check_device_err(ctx, "batched layout (tuning)"))) return rc;
+        cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]);
       }
+      const float ms = std::max(std::min(t[0], t[1]), std::min(std::max(t[0], t[1]), t[2]));
+      if (ms >= 0.97f * best) break;
+      best = ms;
+      best_rows = rows;
     }
     ctx->batch_seg_rows = best_rows;
-    ctx->batch_tuned_shape = shape;
+    ctx->batch_tuned_sizes = sizes;
     ctx->batch_tuned_k = k;
+    ctx->batch_tuned_c = c;
     ctx->batch_tune_ms = best;
     if (ctx->batch_graph) {
       cudaGraphExecDestroy(ctx->batch_graph);
@@ -875,7 +886,7 @@ extern "C" int phde_layout_batched(phde_ctx *ctx, const phde_layout_opts *o, dou
     }
   }
   if ((rc = set_segments(ctx->batch_seg_rows))) return rc;
-  const int64_t launches0 = ctx->launches;
+  const int64_t launches0 = ctx->launches - dist_launches;
   // ---- run: replay the captured graph, or capture it (first call after tuning), or launch directly ----
   const int key_c = c * 8 + o->strategy;  // the captured sequence depends on c and the pivot strategy
   if (ctx->batch_graph && (ctx->batch_graph_c != key_c || ctx->batch_graph_ws != ctx->ws_epoch)) {
@@ -884,7 +895,12 @@ extern "C" int phde_layout_batched(phde_ctx *ctx, const phde_layout_opts *o, dou
   }
   cudaEventRecord(ctx->ev[0], ctx->stream);
   bool replayed = false, ran = false;
-  if (ctx->batch_warm_key != key_c) {
+  if (tune) {  // the distance columns are there
+    if ((rc = batch_dense(ctx, q, k, c))) return rc;
+    ran = true;
+    ctx->batch_warm_key = key_c;
+    ctx->batch_no_graph = false;
+  } else if (ctx->batch_warm_key != key_c) {
     // the first call with this sequence runs it directly (it allocates its buffers); the next one captures it
     if ((rc = batch_pipeline(ctx, q, k, c))) return rc;
     ran = true;
@@ -934,8 +950,9 @@ extern "C" int phde_layout_batched(phde_ctx *ctx, const phde_layout_opts *o, dou
   ull h_edges = 0;
   PHDE_CK(ctx, cudaMemcpyAsync(&h_edges, q.edges, sizeof(ull), cudaMemcpyDeviceToHost, ctx->stream));
   PHDE_CK(ctx, cudaStreamSynchronize(ctx->stream));
-  float ms = 0;
+  float ms = 0, dist_ms = 0;
   cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
+  if (tune) cudaEventElapsedTime(&dist_ms, ctx->ev[4], ctx->ev[5]);
   int naccepted_min = k, ndisc = 0, sweeps = 0;
   for (int b = 0; b < B; b++) {
     naccepted_min = std::min(naccepted_min, st[4 * b]);
@@ -955,7 +972,7 @@ extern "C" int phde_layout_batched(phde_ctx *ctx, const phde_layout_opts *o, dou
     stats->ndiscarded = ndisc;
     stats->eig_iters = sweeps;
     stats->gpu_launches = (int)(ctx->launches - launches0);
-    stats->ms_total = ms;
+    stats->ms_total = ms + dist_ms;
     stats->edges_examined = (int64_t)h_edges;
     stats->batch_graph_replay = replayed ? 1 : 0;
     stats->batch_seg_rows = (int)ctx->batch_seg_rows;

@@ -32,8 +32,8 @@ struct phde_ctx {
   int32_t *d_gid = nullptr;                        // [n]: graph of each vertex
   int32_t *d_order = nullptr;                      // [batch_B]: graphs, largest first
   bool batch_blocks = false;                       // Kcenters with one CTA per graph
-  int64_t batch_tuned_shape = -1;                  // autotuned segment length for this batch shape and k
-  int batch_tuned_k = 0;
+  uint64_t batch_tuned_sizes = 0;                  // autotuned segment length for these graph sizes, k and c
+  int batch_tuned_k = 0, batch_tuned_c = 0;
   int64_t batch_seg_rows = 8192;
   float batch_tune_ms = 0;
   cudaGraphExec_t batch_graph = nullptr;           // the captured batched pipeline

@@ -103,7 +103,7 @@ typedef struct {
   double ms_mmult;   /* Laplacian SpMM + Gram product                                               */
   double ms_eig;     /* k x k eigensolve                                                             */
   double ms_coords;  /* coordinates, normalisation and the copy to the host                          */
-  double ms_total;   /* whole call                                                                   */
+  double ms_total;   /* whole call (phde_layout_batched: without the tuning of a first call)          */
   int64_t edges_examined; /* adjacency entries read by the distance passes                          */
   double ms_dist_kernel;  /* device time of the distance kernel launches alone (events around each launch) */
   int dist_kernel_launches; /* number of distance kernel launches (1 for the Kcenters BFS)           */
@@ -111,7 +111,7 @@ typedef struct {
   int msbfs_levels;         /* levels of those sweeps, summed                                           */
   int batch_graph_replay;   /* phde_layout_batched: 1 when the pipeline ran as one CUDA graph launch     */
   int batch_seg_rows;       /* phde_layout_batched: rows per segment CTA picked by the autotuner         */
-  double ms_batch_tune;     /* phde_layout_batched: the autotuner's best whole-batch time (first call)   */
+  double ms_batch_tune;     /* phde_layout_batched: on the call that tuned, the stages after the distances at that length */
   int64_t sssp_rounds;      /* WParHDE: synchronised relaxation rounds of the SSSP passes, summed        */
   /* learned strategies: PHDE_OUTCOME_*; 0 for the reference's strategies */
   int pivot_outcome;

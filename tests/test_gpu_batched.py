@@ -242,3 +242,37 @@ def test_batch_after_a_refused_batch(monkeypatch, mode):
         cb.upload_batch(good)
         xs, _ = cb.layout_batched(4, 2)
         assert all(np.all(np.isfinite(x)) for x in xs)
+
+
+@pytest.mark.parametrize("mode,strategy", [("union", "Kcenters"), ("blocks", "Kcenters"), ("blocks", "Learned")])
+def test_first_batched_call_counts_its_work_once(monkeypatch, mode, strategy):
+    """The call that tunes the segment length computes the distances once: its counts and layouts are the later
+    calls'."""
+    monkeypatch.setenv("PHDE_BATCH_BFS", mode)
+    with Context(0) as cb:
+        cb.upload_batch([graphs.mesh(40, 30 + i, seed=i) for i in range(5)])
+        x1, s1 = cb.layout_batched(6, 2, strategy=strategy)
+        x1 = [x.copy() for x in x1]
+        assert s1["ms_batch_tune"] > 0
+        for _ in range(3):  # captured, then replayed
+            x, s = cb.layout_batched(6, 2, strategy=strategy)
+            assert s["ms_batch_tune"] == 0 and s["batch_seg_rows"] == s1["batch_seg_rows"]
+            assert s["edges_examined"] == s1["edges_examined"] > 0
+            if strategy == "Kcenters":  # the learned sweep makes its plan of the graphs on the first call
+                assert s["gpu_launches"] == s1["gpu_launches"]
+            for a, b in zip(x1, x):
+                assert np.array_equal(a, b)
+
+
+def test_segment_length_is_tuned_for_the_batch_at_hand():
+    """Batches of equal totals but other graphs, other k or other c do not take over each other's length."""
+    a, b = graphs.mesh(20, 30, seed=1), graphs.mesh(40, 25, seed=2)
+    with Context(0) as cb:
+        cb.upload_batch([a, b])
+        assert cb.layout_batched(6, 2)[1]["ms_batch_tune"] > 0
+        cb.upload_batch([b, a])
+        assert cb.layout_batched(6, 2)[1]["ms_batch_tune"] > 0
+        assert cb.layout_batched(6, 3)[1]["ms_batch_tune"] > 0
+        assert cb.layout_batched(5, 3)[1]["ms_batch_tune"] > 0
+        cb.upload_batch([b, a])
+        assert cb.layout_batched(5, 3)[1]["ms_batch_tune"] == 0
