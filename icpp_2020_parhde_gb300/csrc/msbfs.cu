@@ -140,6 +140,12 @@ __device__ __forceinline__ void ld_front_if(const ull *p, ull (&x)[W], uint64_t 
         "mov.u64 %3, 0;\n\t@p ld.global.cg.L2::cache_hint.v4.u64 {%0, %1, %2, %3}, [%4], %5;\n\t}"
         : "=&l"(x[0]), "=&l"(x[1]), "=&l"(x[2]), "=&l"(x[3])
         : "l"(p), "l"(keep), "r"((uint32_t)on));
+  } else if constexpr (W == 2) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\tmov.u64 %0, 0;\n\tmov.u64 %1, 0;\n\t"
+        "@p ld.global.cg.L2::cache_hint.v2.u64 {%0, %1}, [%2], %3;\n\t}"
+        : "=&l"(x[0]), "=&l"(x[1])
+        : "l"(p), "l"(keep), "r"((uint32_t)on));
   } else {
 #pragma unroll
     for (int w = 0; w < W; w++)
