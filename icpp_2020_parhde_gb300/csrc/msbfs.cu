@@ -1007,14 +1007,17 @@ static int msbfs_run(phde_ctx *ctx, const int64_t *d_src, int nsrc, int nlist, i
   ull *trace = trace_path ? (ull *)phde_buf(ctx, "ms.trace", sizeof(ull) * 2 * trace_cap) : nullptr;
   for (int s0 = 0; s0 < nsrc; s0 += 64 * Wmax) {
     const int ns = std::min(nsrc - s0, 64 * Wmax);
-    const int W = (ns + 63) / 64;
+    // dense levels of index-local graphs stage frontier windows (PHDE_MSBFS_WINDOW=0 or 1 picks outright)
+    const char *we = getenv("PHDE_MSBFS_WINDOW");
+    const bool win = we ? atoi(we) != 0 : ctx->ms_local;
+    // three words are gathered by three requests, four by one: a record sweep of 129 to 192 sources takes the kernel of
+    // four (180 sources: R-MAT 20 2.32 -> 1.96 ms, 1M-vertex 3-D geometric graph 16.0 -> 12.7), but not with windows,
+    // whose copies would grow by a third (200k-vertex 2-D 12.4 against 12.7).  Level arrays keep the words their readers count.
+    const int words = (ns + 63) / 64, W = words == 3 && !lvl && !win ? 4 : words;
     const void *fn = W == 1 ? (const void *)msbfs_kernel<1>
                    : W == 2 ? (const void *)msbfs_kernel<2>
                    : W == 3 ? (const void *)msbfs_kernel<3>
                             : (const void *)msbfs_kernel<4>;
-    // dense levels of index-local graphs stage frontier windows (PHDE_MSBFS_WINDOW=0 or 1 picks outright)
-    const char *we = getenv("PHDE_MSBFS_WINDOW");
-    const bool win = we ? atoi(we) != 0 : ctx->ms_local;
     const size_t dyn = win ? sizeof(ull) * 3 * MS_WIN * W : 0;
     if (int arc = phde_allow_smem(ctx, (const void *)fn)) return arc;
     // with a window, all of the unified L1/shared storage as shared memory (two CTAs per SM); without, the

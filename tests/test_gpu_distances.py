@@ -347,3 +347,16 @@ def test_sssp_on_a_converted_graph(gpu_ctx, hub):
     low = src > g.adj
     gpu_ctx.graph_from_entries(src[low] + 1, g.adj[low] + 1, g.weights[low], g.n, g.n, True)
     assert np.array_equal(gpu_ctx.distances([3])[:, 0], orc.sssp(g, 3))
+
+
+@pytest.mark.parametrize("window", ["0", "1"])
+@pytest.mark.parametrize("nsrc", [65, 128, 129, 180, 192, 193, 400])
+def test_multi_source_bfs_words(gpu_ctx, monkeypatch, nsrc, window):
+    """Sweeps at the edges of the frontier words' counts, a second sweep among them: every column against one source."""
+    monkeypatch.setenv("PHDE_MSBFS_WINDOW", window)
+    g = graphs.rgg(6000, dim=3, avg_degree=10, seed=35)
+    gpu_ctx.upload(g)
+    src = np.random.default_rng(nsrc).integers(0, g.n, size=nsrc)
+    d = gpu_ctx.distances(src)
+    for i in range(nsrc):
+        assert np.array_equal(d[:, i], orc.bfs(g, int(src[i]))), i
