@@ -41,6 +41,11 @@
 namespace {
 
 constexpr int KC_THREADS = 1024;
+constexpr int KC_HISTORY = 4096;  // passes whose history is kept in shared memory
+// Shared memory with the frontier bitmap in it, at most: the copy of a larger bitmap costs a bottom-up level what its
+// reads gain (216 KB against 116, 12 passes: R-MAT 21 1.61 against 1.69 ms, 1.6M-vertex 3-D geometric graph 15.33 against
+// 15.20, 1200 x 1200 mesh 74.9 against 72.1; none against 116: R-MAT 20, 30 passes, 3.07 against 3.00).
+constexpr size_t KC_SMEM = 116 * 1024;
 
 struct KcArgs {
   const int64_t *off;
@@ -62,6 +67,7 @@ struct KcArgs {
   int64_t W;        // words per bitmap
   int smem_bm;      // copy the frontier bitmap into shared memory for bottom-up levels
   int cap;          // entries of the block's list of new vertices: a multiple of KC_THREADS, at least two of them
+  int hist;         // passes whose history is in shared memory
   ull *ctr;         // [4] ring of (count << 32 | edges)
   ull *edges;       // [1] adjacency entries read
   ull *trace;       // optional timeline: per level {globaltimer, pass<<40 | level<<32 | in_bu, frontier count, edges}
@@ -144,8 +150,13 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
   __shared__ unsigned s_listed;
   __shared__ uint32_t s_win[KC_THREADS / 32][32];
   __shared__ ull red[32];
-  extern __shared__ __align__(16) uint32_t s_hist[];  // [P]: every block keeps the same selection history; the list, the bitmap
-  const KcList list{s_hist + ((a.P + 3) & ~3), &s_listed};
+  extern __shared__ __align__(16) uint32_t s_hist[];  // [a.hist]: every block keeps the same history; the list, the bitmap
+  const KcList list{s_hist + ((a.hist + 3) & ~3), &s_listed};
+  // vertex i of the selection history: in shared memory, or (more passes than that is worth) from the passes' outputs
+  auto history = [&](int i) -> uint32_t {
+    if (i < a.hist) return s_hist[i];
+    return a.variant == 2 ? (uint32_t)__ldcg(a.sources + i) : 0xffffffffu - (uint32_t)(__ldcg(a.keys + i) & 0xffffffffull);
+  };
   uint32_t *s_bm = list.v + a.cap;
   const int full = a.cap / KC_THREADS - 1;  // iterations between looks at the list
   if (threadIdx.x == 0) s_listed = 0u;  // barriers of the first pass's start come before its use
@@ -165,7 +176,7 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
     src = a.resume[1];
     level0 = (int32_t)a.resume[2];
     edges0 = a.resume[3];
-    for (int i = tid; i < p0; i += blockDim.x)
+    for (int i = tid; i < min(p0, a.hist); i += blockDim.x)
       s_hist[i] = a.variant == 2 ? (uint32_t)a.sources[i] : 0xffffffffu - (uint32_t)(a.keys[i] & 0xffffffffull);
     __syncthreads();
   }
@@ -470,7 +481,7 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
     const uint32_t raw = 0xffffffffu - (uint32_t)(key & 0xffffffffull);
     const int32_t maxval = (int32_t)(key >> 32);
     int hit = 0;
-    for (int i = tid; i < p; i += blockDim.x) hit |= (s_hist[i] == raw);
+    for (int i = tid; i < p; i += blockDim.x) hit |= (history(i) == raw);
     hit = __syncthreads_or(hit);
     int64_t next = raw;
     if (p >= 1 && hit) {
@@ -479,7 +490,7 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
       for (int64_t v = gbase + tid; v < n; v += gstride) {
         if (a.min_d[v] != maxval) continue;
         bool inh = false;
-        for (int i = 0; i < p && !inh; i++) inh = (s_hist[i] == (uint32_t)v);
+        for (int i = 0; i < p && !inh; i++) inh = (history(i) == (uint32_t)v);
         if (!inh) atomicMax(a.fixkey + p, (ull)v + 1ull);
       }
       ull fk;
@@ -487,7 +498,7 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
       if (fk) next = (int64_t)(fk - 1ull);
     }
     __syncthreads();
-    if (tid == 0) s_hist[p] = a.variant == 2 ? (uint32_t)src : raw;
+    if (tid == 0 && p < a.hist) s_hist[p] = a.variant == 2 ? (uint32_t)src : raw;
     __syncthreads();
     src = next;
   }
@@ -1244,17 +1255,15 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   if ((rc = phde_reset_sync(ctx))) return rc;
 
   int per_sm = 0;
-  // shared memory: the selection history, then (when it fits two blocks per SM) the frontier bitmap
-  const size_t hist_bytes = sizeof(uint32_t) * (size_t)((P + 3) & ~3);
-  const size_t bm_bytes = sizeof(uint32_t) * (size_t)W;
-  // ... and the list of new vertices, 4096 entries, or 2048 beside the largest bitmaps
-  const int smem_bm = hist_bytes + bm_bytes <= 98 * 1024;
-  const int cap = smem_bm && hist_bytes + bm_bytes > 90 * 1024 ? 2 * KC_THREADS : 4 * KC_THREADS;
-  const size_t smem = hist_bytes + sizeof(uint32_t) * cap + (smem_bm ? bm_bytes : 0);
+  // shared memory: the selection history, the list of new vertices, then the frontier bitmap up to KC_SMEM; one block per
+  // SM (its registers are the SM's)
+  const int hist = std::min(P, KC_HISTORY), cap = 4 * KC_THREADS;
+  const size_t fixed = sizeof(uint32_t) * (size_t)(((hist + 3) & ~3) + cap), bm_bytes = sizeof(uint32_t) * (size_t)W;
+  const int smem_bm = fixed + bm_bytes <= KC_SMEM;
+  const size_t smem = fixed + (smem_bm ? bm_bytes : 0);
   if (int arc = phde_allow_smem(ctx, (const void *)kcenters_bfs_kernel)) return arc;
   PHDE_CK(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kcenters_bfs_kernel, KC_THREADS, smem));
   if (per_sm < 1) return phde_fail(ctx, PHDE_ERR_CUDA, "kcenters kernel cannot be resident");
-  per_sm = std::min(per_sm, 2);
   KcArgs a;
   a.off = ctx->d_off;
   a.adj = ctx->d_adj;
@@ -1287,6 +1296,7 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   a.W = W;
   a.smem_bm = smem_bm;
   a.cap = cap;
+  a.hist = hist;
   a.edges = d_edges;
   // PHDE_BFS_TRACE=<file>: write the per-level timeline of this launch as CSV after it completes
   const char *trace_file = getenv("PHDE_BFS_TRACE");
@@ -1310,7 +1320,7 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   a.resume = nullptr;
   // a traced call keeps every pass in the kernel that writes the timeline
   if (B == 0 && !a.trace && (rc = run_cluster_passes(ctx, a))) return rc;
-  PHDE_CK(ctx, cudaLaunchCooperativeKernel((const void *)kcenters_bfs_kernel, dim3(ctx->nsm * per_sm),
+  PHDE_CK(ctx, cudaLaunchCooperativeKernel((const void *)kcenters_bfs_kernel, dim3(ctx->nsm),
                                            dim3(KC_THREADS), args, smem, ctx->stream));
   PHDE_LAUNCHED(ctx);
   cudaEventRecord(ctx->kev[1], ctx->stream);

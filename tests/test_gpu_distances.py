@@ -360,3 +360,23 @@ def test_multi_source_bfs_words(gpu_ctx, monkeypatch, nsrc, window):
     d = gpu_ctx.distances(src)
     for i in range(nsrc):
         assert np.array_equal(d[:, i], orc.bfs(g, int(src[i]))), i
+
+
+@pytest.mark.parametrize("leaves", [802_000, 818_000, 820_000])
+def test_kcenters_bitmaps_around_the_shared_memory_limit(gpu_ctx, leaves):
+    """Bottom-up levels whose frontier bitmap just fits the block's shared memory beside the list, and does not."""
+    g = graphs.star_graph(leaves)
+    gpu_ctx.upload(g)
+    D, s = gpu_ctx.kcenters(3, 0)
+    Do, so = orc.kcenters(g, 3, 0, parallel=True)
+    assert np.array_equal(s, so) and np.array_equal(D, Do)
+
+
+@pytest.mark.parametrize("variant", [0, 2])
+@pytest.mark.parametrize("passes", [4096, 4097, 56_000])
+def test_kcenters_with_a_long_history(gpu_ctx, passes, variant):
+    """Passes at and past those whose history is in shared memory, and more than shared memory holds."""
+    g = graphs.path_graph(9)
+    gpu_ctx.upload(g)
+    _, s = gpu_ctx.kcenters(passes, variant, want_dist=False)
+    assert np.array_equal(s, orc.kcenters(g, passes, variant)[1])
