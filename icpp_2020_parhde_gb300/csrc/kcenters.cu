@@ -1037,7 +1037,8 @@ __global__ void __launch_bounds__(KL_THREADS, 1) kcenters_cluster_kernel(KlArgs 
           const uint2 row = kl_row(l, y);
           list[at] = row;
           longrow |= row.y > KL_ROW;
-          asm volatile("prefetch.global.L1 [%0];" ::"l"(a.adj + row.x));  // read after the block's barrier
+          // read after the block's barrier; an empty row may start past the array (a directed graph's last vertices)
+          if (row.y) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.adj + row.x));
         }
         if (longrow) s_long[par] = 1u;
       }

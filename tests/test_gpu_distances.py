@@ -380,3 +380,21 @@ def test_kcenters_with_a_long_history(gpu_ctx, passes, variant):
     gpu_ctx.upload(g)
     _, s = gpu_ctx.kcenters(passes, variant, want_dist=False)
     assert np.array_equal(s, orc.kcenters(g, passes, variant)[1])
+
+
+def test_cluster_search_reaches_empty_rows_at_the_end(gpu_ctx):
+    """A directed CSR whose last vertices have no neighbours: their rows start past an adjacency of whole pages."""
+    spine, width = 512, 1024
+    nnz = spine * width  # 2 MiB of adjacency
+    nxt = np.arange(1, spine)
+    rows, first = [], spine
+    for i in range(spine):
+        leaves = width if i == spine - 1 else width - 1
+        rows.append(np.concatenate([nxt[i: i + 1], np.arange(first, first + leaves)]))
+        first += leaves
+    off = np.concatenate([np.arange(spine + 1) * width, np.full(first - spine, nnz)])
+    g = CSRGraph(off.astype(np.uint32), np.concatenate(rows).astype(np.uint32))
+    gpu_ctx.upload(g)
+    d = gpu_ctx.distances([0])[:, 0]
+    want = np.concatenate([np.arange(spine)] + [np.full(len(r) - (i < spine - 1), i + 1) for i, r in enumerate(rows)])
+    assert np.array_equal(d, want)
