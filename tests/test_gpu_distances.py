@@ -398,3 +398,27 @@ def test_cluster_search_reaches_empty_rows_at_the_end(gpu_ctx):
     d = gpu_ctx.distances([0])[:, 0]
     want = np.concatenate([np.arange(spine)] + [np.full(len(r) - (i < spine - 1), i + 1) for i, r in enumerate(rows)])
     assert np.array_equal(d, want)
+
+
+@pytest.mark.parametrize("more", [-1, 0, 1, 155])
+def test_top_down_levels_around_one_grid_iteration(gpu_ctx, monkeypatch, tmp_path, more):
+    """Top-down levels with as many out-edges as the grid has threads, one fewer and more: pushed at once, or listed
+    first.  A hub with that many neighbours and then its leaves, before a mesh large enough to keep both levels
+    top-down; the traced search stays on the grid and says so."""
+    import torch
+    width = torch.cuda.get_device_properties(0).multi_processor_count * 1024 + more
+    body = graphs.mesh(700, 700, seed=36)
+    src = np.repeat(np.arange(body.n), np.diff(body.offsets.astype(np.int64)))
+    keep = src < body.adj
+    first = width + 1  # vertices: the source, the hub, width - 1 leaves, the mesh behind the last leaf
+    lo = np.concatenate([[0], np.full(width - 1, 1), [width], src[keep] + first])
+    hi = np.concatenate([[1], np.arange(2, width + 1), [first], body.adj[keep].astype(np.int64) + first])
+    g = graphs._csr_from_undirected(first + body.n, lo, hi)
+    trace = tmp_path / "levels.csv"
+    monkeypatch.setenv("PHDE_BFS_TRACE", str(trace))
+    gpu_ctx.upload(g)
+    D, _ = gpu_ctx.kcenters(1, 0)
+    assert np.array_equal(D[:, 0], orc.bfs(g, 0))
+    level = [[int(x) for x in line.split(",")] for line in trace.read_text().splitlines()[1:4]]
+    assert [(r[3], r[4]) for r in level] == [(0, 0), (1, 0), (2, 0)]  # none of the three is bottom-up
+    assert (level[0][5], level[0][6]) == (1, width) and (level[1][5], level[1][6]) == (width - 1, width)

@@ -41,3 +41,34 @@ def test_ordered_sums_bitwise(gpu_ctx, algo, make, k):
             X[:, t] = X[:, t] + C[:, j] * y[j]
         X[:, t] *= 1.0 / np.sqrt(np.add.accumulate(X[:, t] * X[:, t])[-1])
     assert np.array_equal(r.coords, X)
+
+
+def comet(n: int, tail: int):
+    """A path of `tail` vertices, numbered from its far end, to a hub with the other vertices as leaves: the first terms
+    of the sums are the large ones, so that the rest of a sum stays in one binade."""
+    lo = np.concatenate([np.arange(tail), np.full(n - tail - 1, tail)])
+    hi = np.concatenate([np.arange(1, tail + 1), np.arange(tail + 1, n)])
+    return graphs._csr_from_undirected(n, lo, hi)
+
+
+@pytest.mark.parametrize("algo", ["PivotMDS", "PHDE"])
+@pytest.mark.parametrize("n,tail", [(n, 12) for n in (31, 32, 33)] +
+                         [(n, 30) for n in (1055, 1056, 1057, 1087, 1088, 1089, 2079, 2080, 2081)])
+def test_ordered_sums_at_the_chunks_edges(gpu_ctx, algo, n, tail):
+    """A sum starts with 32 terms one by one and goes on in chunks of 1024: sums that end there, one term before and one
+    after, and 32 terms later."""
+    g = comet(n, tail)
+    gpu_ctx.upload(g)
+    k = 3
+    r = gpu_ctx.layout(algo, "Kcenters", k=k, c=2, eig="exact", extra=True)
+    C = r.basis
+    assert np.array_equal(C, orc.layout(g, algo, "Kcenters", k, 2, eig="exact", nthreads=1).S)
+    want = np.array([[np.add.accumulate(C[:, p] * C[:, q])[-1] for q in range(k)] for p in range(k)])
+    assert np.array_equal(r.gram, want)
+    X = np.zeros((n, 2))
+    for t in range(2):
+        y = r.evecs[:, k - 1 - t]
+        for j in range(k):
+            X[:, t] = X[:, t] + C[:, j] * y[j]
+        X[:, t] *= 1.0 / np.sqrt(np.add.accumulate(X[:, t] * X[:, t])[-1])
+    assert np.array_equal(r.coords, X)
