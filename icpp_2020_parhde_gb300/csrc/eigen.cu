@@ -1059,7 +1059,10 @@ int phde_eigensolve(phde_ctx *ctx, const double *d_M, int N, int c, int largest,
     const int NO = (N + PW_CL - 1) / PW_CL;
     const size_t csmem = sizeof(double) * ((size_t)N * N + 2 * (size_t)NO * N + 2 * (N + 1) + NO + 1);
     double *start = (double *)phde_buf(ctx, "eig.start", sizeof(double) * N * N);
-    if (!start) return PHDE_ERR_OOM;
+    if (!start) {
+      ctx->eig_start = 0;  // the smaller buffer is gone as well, and its address may come back
+      return PHDE_ERR_OOM;
+    }
     if (ctx->eig_start < N * N || ctx->eig_start_buf != start) {  // the same for every solve: kept in the context
       const std::vector<double> h = start_vectors(N * N);
       PHDE_CK(ctx, cudaMemcpyAsync(start, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, ctx->stream));
