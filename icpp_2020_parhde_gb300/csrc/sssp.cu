@@ -627,10 +627,11 @@ int phde_run_sssp(phde_ctx *ctx, const int64_t *d_src, int32_t *d_col, int32_t d
   PHDE_CK(ctx, cudaMemsetAsync(minfar, 0xff, sizeof(ull) * 2, ctx->stream));
   if ((rc = phde_reset_sync(ctx))) return rc;
   // Resident CTAs per SM: one (with the registers it wants) on small graphs, whose rounds are short, two (registers
-  // capped at 32) on larger ones; PHDE_SSSP_CTAS=1 or 2 picks outright.  Lane groups change over at 2^18 vertices
-  // (65 x 61 x 70 grid, layout: 23.7 ms with two, 24.6 with one; 300k-vertex geometric graph of degree 8: 44 against
-  // 49), the edge-balanced kernel at 2^20 (64^3 grid: 1.5 ms per pass with one against 2.1; 256^3: 14.3 with two
-  // against 16.1).
+  // capped at 32) on larger ones; PHDE_SSSP_CTAS=1 or 2 picks outright.  Lane groups change over at 2^18 vertices, where
+  // grids cross (four passes with one and two, ms: 52^3 2.85 and 3.13, 58^3 3.48 and 3.51, 63^3 4.22 and 4.17, 72^3 5.23
+  // and 4.89; a 600 x 600 mesh 20.5 and 20.8, longer rows cross lower: 200k vertices in 2-D 17.8 and 17.1, in 3-D 7.6 and
+  // 5.7), the edge-balanced kernel at 2^20 (64^3 grid: 1.5 ms per pass with one against 2.1; 256^3: 14.3 with two against
+  // 16.1).
   const char *ce = getenv("PHDE_SSSP_CTAS");
   const int want = ce ? (atoi(ce) == 1 ? 1 : 2) : (n < ((int64_t)1 << (group ? 18 : 20)) ? 1 : 2);
   const void *kfn = want == 1 ? (const void *)sssp_nearfar_kernel<1> : (const void *)sssp_nearfar_kernel<2>;

@@ -104,7 +104,8 @@ typedef struct {
   double ms_eig;     /* k x k eigensolve                                                             */
   double ms_coords;  /* coordinates, normalisation and the copy to the host                          */
   double ms_total;   /* whole call (phde_layout_batched: without the tuning of a first call)          */
-  int64_t edges_examined; /* adjacency entries read by the distance passes                          */
+  int64_t edges_examined; /* adjacency entries read by the distance passes: every row once a pass where a search runs
+                             on one cluster or CTA; the whole grid stops a row at its first hit in bottom-up levels */
   double ms_dist_kernel;  /* device time of the distance kernel launches alone (events around each launch) */
   int dist_kernel_launches; /* number of distance kernel launches (1 for the Kcenters BFS)           */
   double ms_msbfs_kernel;   /* of which multi-source BFS sweeps (learned and random strategies)          */
