@@ -969,11 +969,10 @@ __global__ void __launch_bounds__(KL_THREADS, 1) kcenters_cluster_kernel(KlArgs 
     if (tid == 0 && rank == 0) a.sources[p] = src;
     cluster_barrier();  // every CTA's words are clear
     l.cnt = mine ? 1u : 0u;
-    uint32_t L = 0, before = 0;  // before: `edges` of the levels before L
+    uint32_t L = 0;
     bool wide = false;
     for (;;) {
       const uint32_t par = L & 1;
-      before = edges;
       l.next = next_s + par * 4u * words;
       // ---- expand ----
       if (tid == 0) {  // for the scan after the barrier; what the last scan left is in the other place
@@ -1037,17 +1036,24 @@ __global__ void __launch_bounds__(KL_THREADS, 1) kcenters_cluster_kernel(KlArgs 
           const uint2 row = kl_row(l, y);
           list[at] = row;
           longrow |= row.y > KL_ROW;
-          // read after the block's barrier; an empty row may start past the array (a directed graph's last vertices)
-          if (row.y) asm volatile("prefetch.global.L1 [%0];" ::"l"(a.adj + row.x));
+          // read after the block's barrier; an empty row may start past the array (a directed graph's last vertices): a
+          // select, as a branch here is 2 % of a geometric graph's passes
+          asm volatile("prefetch.global.L1 [%0];" ::"l"(a.adj + (row.y ? row.x : 0u)));
         }
         if (longrow) s_long[par] = 1u;
       }
       __syncthreads();
       l.cnt = *(volatile uint32_t *)&s_cnt[par];
     }
-    edges_all += before;  // of a finished pass all: its last level found nothing
+    edges_all += edges;
     if (wide) {  // leave the rest of the pass to the whole grid, which expands level L again
-      const ull e = block_sum((ull)before, red);
+      ull e = edges;  // summed modulo 2^64: without the rows of level L, which a CTA expanded where its list held them
+      if (l.cnt <= KL_LIST)
+        for (uint32_t i = tid; i < l.cnt; i += KL_THREADS) {
+          e -= list[i].y;
+          edges_all -= list[i].y;
+        }
+      e = block_sum(e, red);
       if (tid == 0) atomicAdd((ull *)a.resume + 3, e);
       if (tid == 0 && rank == 0) {
         a.resume[0] = p;
