@@ -41,7 +41,7 @@
 namespace {
 
 constexpr int KC_THREADS = 1024;
-constexpr int KC_HISTORY = 4096;  // passes whose history is kept in shared memory
+constexpr int KC_HISTORY = 4096;  // passes whose history is kept in shared memory, at most
 // Shared memory with the frontier bitmap in it, at most: the copy of a larger bitmap costs a bottom-up level what its
 // reads gain (216 KB against 116, 12 passes: R-MAT 21 1.61 against 1.69 ms, 1.6M-vertex 3-D geometric graph 15.33 against
 // 15.20, 1200 x 1200 mesh 74.9 against 72.1; none against 116: R-MAT 20, 30 passes, 3.07 against 3.00).
@@ -67,7 +67,7 @@ struct KcArgs {
   int64_t W;        // words per bitmap
   int smem_bm;      // copy the frontier bitmap into shared memory for bottom-up levels
   int cap;          // entries of the block's list of new vertices: a multiple of KC_THREADS, at least two of them
-  int hist;         // passes whose history is in shared memory
+  uint32_t *hist;   // [grid x P] selection histories of the blocks when they are not in shared memory
   ull *ctr;         // [4] ring of (count << 32 | edges)
   ull *edges;       // [1] adjacency entries read
   ull *trace;       // optional timeline: per level {globaltimer, pass<<40 | level<<32 | in_bu, frontier count, edges}
@@ -150,13 +150,10 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
   __shared__ unsigned s_listed;
   __shared__ uint32_t s_win[KC_THREADS / 32][32];
   __shared__ ull red[32];
-  extern __shared__ __align__(16) uint32_t s_hist[];  // [a.hist]: every block keeps the same history; the list, the bitmap
-  const KcList list{s_hist + ((a.hist + 3) & ~3), &s_listed};
-  // vertex i of the selection history: in shared memory, or (more passes than that is worth) from the passes' outputs
-  auto history = [&](int i) -> uint32_t {
-    if (i < a.hist) return s_hist[i];
-    return a.variant == 2 ? (uint32_t)__ldcg(a.sources + i) : 0xffffffffu - (uint32_t)(__ldcg(a.keys + i) & 0xffffffffull);
-  };
+  extern __shared__ __align__(16) uint32_t kc_smem[];  // the selection history, the list, the bitmap
+  // every block keeps the same history: [P] in shared memory, or for very many passes each block's own in global memory
+  uint32_t *s_hist = a.hist ? a.hist + (int64_t)blockIdx.x * a.P : kc_smem;
+  const KcList list{kc_smem + (a.hist ? 0 : (a.P + 3) & ~3), &s_listed};
   uint32_t *s_bm = list.v + a.cap;
   const int full = a.cap / KC_THREADS - 1;  // iterations between looks at the list
   if (threadIdx.x == 0) s_listed = 0u;  // barriers of the first pass's start come before its use
@@ -168,15 +165,11 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
   uint32_t step = 0;
   ull edges_local = 0;
   int p0 = 0;
-  int32_t level0 = 0;  // levels of pass p0 that are done
-  int64_t edges0 = 0;  // and the edges that left them
   if (a.resume) {  // go on where the cluster stopped: the same history, from the passes' keys or sources
     p0 = (int)a.resume[0];
     if (p0 >= a.P) return;
     src = a.resume[1];
-    level0 = (int32_t)a.resume[2];
-    edges0 = a.resume[3];
-    for (int i = tid; i < min(p0, a.hist); i += blockDim.x)
+    for (int i = tid; i < p0; i += blockDim.x)
       s_hist[i] = a.variant == 2 ? (uint32_t)a.sources[i] : 0xffffffffu - (uint32_t)(a.keys[i] & 0xffffffffull);
     __syncthreads();
   }
@@ -186,8 +179,14 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
     int64_t s_off = 0;
     uint32_t sdeg = 0;
     uint32_t f_cnt = 1, f_edges = 0;
-    const bool mid = p == p0 && level0 > 0;  // a pass that the cluster began
-    if (mid) {  // its last level, read back from the column, is the frontier (step is 0)
+    int64_t edges_to_check = a.nnz;
+    int32_t L = 0;
+    if (a.resume && p == (int)a.resume[0] && a.resume[2] > 0) {
+      // a pass that the cluster began: its last level, read back from the column, is the frontier (step is 0).  Where it
+      // stopped is read here again: kept in registers across the passes, it cost every level (1 % of a batch's union).
+      const int32_t level0 = (int32_t)a.resume[2];
+      L = level0;
+      edges_to_check -= a.resume[3];
       const bool once = n <= gstride;
       int since = 0;
       for (int64_t base = gbase; base < n; base += gstride) {
@@ -257,10 +256,9 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
       f_cnt = (uint32_t)(q >> 32);
       f_edges = (uint32_t)(q & 0xffffffffull);
     }
-    int64_t edges_to_check = mid ? a.nnz - edges0 : a.nnz, scout = f_edges;
+    int64_t scout = f_edges;
     bool in_bu = false;
     int64_t awake = 0, old_awake = 0;
-    int32_t L = mid ? level0 : 0;
 
     while (f_cnt > 0) {
       if (!in_bu) {
@@ -481,7 +479,7 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
     const uint32_t raw = 0xffffffffu - (uint32_t)(key & 0xffffffffull);
     const int32_t maxval = (int32_t)(key >> 32);
     int hit = 0;
-    for (int i = tid; i < p; i += blockDim.x) hit |= (history(i) == raw);
+    for (int i = tid; i < p; i += blockDim.x) hit |= (s_hist[i] == raw);
     hit = __syncthreads_or(hit);
     int64_t next = raw;
     if (p >= 1 && hit) {
@@ -490,7 +488,7 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
       for (int64_t v = gbase + tid; v < n; v += gstride) {
         if (a.min_d[v] != maxval) continue;
         bool inh = false;
-        for (int i = 0; i < p && !inh; i++) inh = (history(i) == (uint32_t)v);
+        for (int i = 0; i < p && !inh; i++) inh = (s_hist[i] == (uint32_t)v);
         if (!inh) atomicMax(a.fixkey + p, (ull)v + 1ull);
       }
       ull fk;
@@ -498,7 +496,7 @@ __global__ void __launch_bounds__(KC_THREADS) kcenters_bfs_kernel(KcArgs a) {
       if (fk) next = (int64_t)(fk - 1ull);
     }
     __syncthreads();
-    if (tid == 0 && p < a.hist) s_hist[p] = a.variant == 2 ? (uint32_t)src : raw;
+    if (tid == 0) s_hist[p] = a.variant == 2 ? (uint32_t)src : raw;
     __syncthreads();
     src = next;
   }
@@ -1264,8 +1262,14 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   int per_sm = 0;
   // shared memory: the selection history, the list of new vertices, then the frontier bitmap up to KC_SMEM; one block per
   // SM (its registers are the SM's)
-  const int hist = std::min(P, KC_HISTORY), cap = 4 * KC_THREADS;
-  const size_t fixed = sizeof(uint32_t) * (size_t)(((hist + 3) & ~3) + cap), bm_bytes = sizeof(uint32_t) * (size_t)W;
+  const int cap = 4 * KC_THREADS;
+  uint32_t *hist = nullptr;
+  if (P > KC_HISTORY) {
+    hist = (uint32_t *)phde_buf(ctx, "kc.hist", sizeof(uint32_t) * (size_t)P * ctx->nsm);
+    if (!hist) return PHDE_ERR_OOM;
+  }
+  const size_t fixed = sizeof(uint32_t) * (size_t)((hist ? 0 : (P + 3) & ~3) + cap);
+  const size_t bm_bytes = sizeof(uint32_t) * (size_t)W;
   const int smem_bm = fixed + bm_bytes <= KC_SMEM;
   const size_t smem = fixed + (smem_bm ? bm_bytes : 0);
   if (int arc = phde_allow_smem(ctx, (const void *)kcenters_bfs_kernel)) return arc;
@@ -1327,8 +1331,8 @@ int phde_run_bfs_passes(phde_ctx *ctx, int P, int variant, const int64_t *d_fixe
   a.resume = nullptr;
   // a traced call keeps every pass in the kernel that writes the timeline
   if (B == 0 && !a.trace && (rc = run_cluster_passes(ctx, a))) return rc;
-  PHDE_CK(ctx, cudaLaunchCooperativeKernel((const void *)kcenters_bfs_kernel, dim3(ctx->nsm),
-                                           dim3(KC_THREADS), args, smem, ctx->stream));
+  PHDE_CK(ctx, cudaLaunchCooperativeKernel((const void *)kcenters_bfs_kernel, dim3(ctx->nsm), dim3(KC_THREADS), args,
+                                           smem, ctx->stream));
   PHDE_LAUNCHED(ctx);
   cudaEventRecord(ctx->kev[1], ctx->stream);
   ctx->kev_pending = true;
