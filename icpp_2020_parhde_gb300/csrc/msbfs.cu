@@ -1035,8 +1035,9 @@ static int msbfs_run(phde_ctx *ctx, const int64_t *d_src, int nsrc, int nlist, i
     PHDE_CK(ctx, cudaMemsetAsync(bms, 0, sizeof(uint32_t) * nw32, ctx->stream));
     PHDE_CK(ctx, cudaMemsetAsync(fbm, 0, sizeof(uint32_t) * 3 * nw32, ctx->stream));
     PHDE_CK(ctx, cudaMemsetAsync(stamp, 0, sizeof(int32_t) * n, ctx->stream));
-    int rc = phde_reset_sync(ctx);
-    if (rc) return rc;
+    // a sweep inside a sequence without host waits keeps the error word: what its warm start found is read at the end
+    PHDE_CK(ctx, cudaMemsetAsync(ctx->d_sync, 0, sizeof(GridSync), ctx->stream));
+    if (sync) PHDE_CK(ctx, cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
     MsArgs a;
     a.off = ctx->d_off;
     a.adj = ctx->d_adj;
@@ -1091,7 +1092,7 @@ static int msbfs_run(phde_ctx *ctx, const int64_t *d_src, int nsrc, int nlist, i
       ctx->kev_pending = false;
       continue;
     }
-    if ((rc = phde_check_device_err(ctx, "multi-source BFS"))) return rc;  // synchronises, collects the time
+    if (int rc = phde_check_device_err(ctx, "multi-source BFS")) return rc;  // synchronises, collects the time
     ctx->msbfs_ms += ctx->kernel_ms - before;
     int nlev = 0;
     PHDE_CK(ctx, cudaMemcpyAsync(&nlev, levels, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));

@@ -276,3 +276,22 @@ def test_segment_length_is_tuned_for_the_batch_at_hand():
         assert cb.layout_batched(5, 3)[1]["ms_batch_tune"] > 0
         cb.upload_batch([b, a])
         assert cb.layout_batched(5, 3)[1]["ms_batch_tune"] == 0
+
+
+@pytest.mark.parametrize("mode", ["union", "blocks"])
+@pytest.mark.parametrize("strategy", ["Kcenters", "Learned"])
+def test_batch_with_a_small_component_apart_is_refused(monkeypatch, mode, strategy):
+    """Both pivot strategies say that a graph is not connected, also when all but a few of its vertices are."""
+    monkeypatch.setenv("PHDE_BATCH_BFS", mode)
+    g = graphs.mesh(40, 30, seed=7)
+    src = np.repeat(np.arange(g.n), np.diff(g.offsets.astype(np.int64)))
+    keep = src < g.adj
+    apart = graphs._csr_from_undirected(g.n + 3, np.concatenate([src[keep], g.n + np.arange(2)]),
+                                        np.concatenate([g.adj[keep].astype(np.int64), g.n + 1 + np.arange(2)]))
+    with Context(0) as cb:
+        cb.upload_batch([graphs.mesh(30, 20, seed=1), apart])
+        with pytest.raises(ParHDEError, match="not connected"):
+            cb.layout_batched(6, 2, strategy=strategy)
+        cb.upload_batch([graphs.mesh(30, 20, seed=1), g])
+        xs, _ = cb.layout_batched(6, 2, strategy=strategy)
+        assert all(np.all(np.isfinite(x)) for x in xs)
