@@ -29,7 +29,7 @@
 // the history, the duplicate fix-up takes the highest-index vertex with the same min_d that is not.
 //
 // Three kernels share that rule and give the same bits.  kcenters_bfs_kernel is the grid-wide one above.
-// kcenters_cluster_kernel runs the passes of a sparse graph whose visited bitmap fits a cluster's shared memory:
+// kcenters_cluster_kernel runs the passes of a sparse graph of up to 3 << 20 vertices in one cluster's shared memory:
 // its levels are a few hundred vertices, so the grid barrier was most of their time.  kcenters_block_kernel gives
 // every graph of a large batch its own CTA.
 #include <cstdio>
